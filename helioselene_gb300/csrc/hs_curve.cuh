@@ -111,7 +111,7 @@ struct Group {
         M = F::add(F::dbl(M), M);
         Xyzz r;
         r.X = F::sub(F::sqr(M), F::dbl(S));
-        r.Y = F::sub(F::mul(M, F::sub(S, r.X)), F::mul(W, y));
+        r.Y = F::mul_sub(M, F::sub(S, r.X), W, y);
         r.ZZ = V;
         r.ZZZ = W;
         if (F::is_zero(r.ZZ))
@@ -141,7 +141,7 @@ struct Group {
         Fe PPP = F::mul(P, PP);
         Fe Q = F::mul(acc.X, PP);
         Fe X3 = F::sub(F::sub(F::sqr(R), PPP), F::dbl(Q));
-        Fe Y3 = F::sub(F::mul(R, F::sub(Q, X3)), F::mul(acc.Y, PPP));
+        Fe Y3 = F::mul_sub(R, F::sub(Q, X3), acc.Y, PPP);
         acc.ZZ = F::mul(acc.ZZ, PP);
         acc.ZZZ = F::mul(acc.ZZZ, PPP);
         acc.X = X3;

@@ -602,7 +602,7 @@ __global__ void __launch_bounds__(RED_CHUNK_THREADS) k_window_chunks(const uint4
                                                                     uint4 *__restrict__ outC, int wide)
 {
     using G = Group<C>;
-    __shared__ uint4 sh[RED_CHUNK_THREADS * 8];
+    __shared__ uint4 sh[RED_CHUNK_THREADS * 8], sa[RED_CHUNK_THREADS * 8];
     const uint32_t ch = blockIdx.x, i = threadIdx.x;
     const uint32_t mi = find_msm(M, ch, [&](uint32_t k) { return desc[k].chunk_base; });
     const MsmDesc d = desc[mi];
@@ -615,13 +615,19 @@ __global__ void __launch_bounds__(RED_CHUNK_THREADS) k_window_chunks(const uint4
     const uint32_t P = nt / q;
     const uint32_t local = ch - d.chunk_base;
     const uint32_t k = local / nbk, b = local % nbk;
-    Xyzz a = G::inf(), r = G::inf(), w = G::inf();
+    Xyzz r = G::inf(), w = G::inf();
     if (i < P) {
         const size_t lo = (size_t)d.group_base + (size_t)k * d.T + (size_t)b * RED_CHUNK + (size_t)i * q;
+        // a_i waits in shared memory: with it, r and w in registers across the
+        // calls the kernel spills
+        Xyzz a = G::inf();
         for (int u = (int)q - 1; u >= 0; u--) {
-            Xyzz t = load_xyzz(in + 16 * (lo + u));
+            const Xyzz t = load_xyzz(in + 16 * (lo + u));
             l2_add<C>(&a, &a, &t);
-            t = load_xyzz(in + 16 * (lo + u) + 8);
+        }
+        st_soa(sa, i, RED_CHUNK_THREADS, a);
+        for (int u = (int)q - 1; u >= 0; u--) {
+            const Xyzz t = load_xyzz(in + 16 * (lo + u) + 8);
             l2_add<C>(&r, &r, &t);
             if (u > 0)
                 l2_add<C>(&w, &w, &r);
@@ -634,7 +640,10 @@ __global__ void __launch_bounds__(RED_CHUNK_THREADS) k_window_chunks(const uint4
     l2_add<C>(&v, &v, &w);
     for (uint32_t m = d.m0; m > 1; m >>= 1)
         l2_dbl<C>(&v, &v);
-    l2_add<C>(&v, &v, &a);
+    if (i < P) {
+        const Xyzz a = ld_soa(sa, i, RED_CHUNK_THREADS);
+        l2_add<C>(&v, &v, &a);
+    }
     block_tree_sum<C>(sh, RED_CHUNK_THREADS, v, i, P);
     if (i == 0) {
         if (DIRECT) {
@@ -891,7 +900,7 @@ struct LaneHorner {
     __device__ __forceinline__ void st(int slot, uint32_t v) const { sl[slot][lane] = v; }
 
     // set s -> set s ^ 1 (the total is not the identity)
-    __device__ void dbl(int s)
+    __device__ __forceinline__ void dbl(int s)
     {
         const int o = s * LSET, n = (s ^ 1) * LSET;
         if (warp == 0) {
@@ -931,7 +940,7 @@ struct LaneHorner {
 
     // set s += addend slots (neither is the identity): 0 -> the sum in set s ^ 1,
     // 1 -> the operands are equal (the caller doubles), 2 -> they cancel
-    __device__ int add(int s, int *flag)
+    __device__ __forceinline__ int add(int s, int *flag)
     {
         const int o = s * LSET, n = (s ^ 1) * LSET;
         if (warp == 0) {
@@ -987,7 +996,7 @@ struct LaneHorner {
 
 // one block of four warps per MSM of the batch
 template <class C>
-__global__ void __launch_bounds__(128) k_combine(const uint4 *__restrict__ S, const MsmDesc *__restrict__ desc,
+__global__ void __launch_bounds__(128, 1) k_combine(const uint4 *__restrict__ S, const MsmDesc *__restrict__ desc,
                                                 uint32_t *__restrict__ out)
 {
     using F = typename C::F;
