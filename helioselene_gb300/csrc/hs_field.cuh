@@ -672,7 +672,9 @@ struct Field {
     // where the division by 2^30 is made exact by adding a multiple of m.  At the
     // end a^-1 = +-d.  A 256-bit input needs at most 590 divsteps (20 batches);
     // the loop is capped at 40.  Against Fermat's a^(m-2) (255 dependent
-    // squarings) the dependent chain is about a tenth as long.
+    // squarings) the dependent chain is about a tenth as long.  Within a batch,
+    // runs of even steps are one shift, and runs of steps without a swap one
+    // multiple of f (below): about a quarter as many turns as steps.
     struct L30 {
         int32_t l[9];  // value = sum l[i] 2^(30 i); l[0..7] in [0, 2^30), l[8] signed
     };
@@ -733,29 +735,38 @@ struct Field {
             uint32_t fl = (uint32_t)f.l[0] | ((uint32_t)f.l[1] << 30);
             uint32_t gl = (uint32_t)g.l[0] | ((uint32_t)g.l[1] << 30);
             int32_t u = 1, v = 0, q = 0, r = 1;
-#pragma unroll 1
-            for (int i = 0; i < 30; i++) {
-                if (D > 0 && (gl & 1u)) {
-                    D = 2 - D;
+            int left = 30;
+            for (;;) {
+                // the even steps up to the next odd g
+                const int z = __ffs((int)(gl | (1u << left))) - 1;
+                gl >>= z;
+                u = (int32_t)((uint32_t)u << z);
+                v = (int32_t)((uint32_t)v << z);
+                D += 2 * z;
+                left -= z;
+                if (left == 0)
+                    break;
+                if (D > 0) {  // the swap of a first-form step: what remains is g + f, halved
                     const uint32_t t = fl;
-                    fl = gl;
-                    gl -= t;
                     const int32_t tu = u, tv = v;
+                    D = -D;
+                    fl = gl;
+                    gl = 0u - t;
                     u = q;
                     v = r;
-                    q -= tu;
-                    r -= tv;
-                } else if (gl & 1u) {
-                    D = 2 + D;
-                    gl += fl;
-                    q += u;
-                    r += v;
-                } else {
-                    D = 2 + D;
+                    q = -tu;
+                    r = -tv;
                 }
-                gl >>= 1;
-                u *= 2;
-                v *= 2;
+                // no swap is due for (1 - D) / 2 steps: of these, up to six at once, by
+                // the multiple w f that clears as many low bits of g (the halvings
+                // are the next turn's even steps).  f (2 - f^2) = 1/f mod 64.
+                int lim = (1 - D) >> 1;
+                lim = lim < left ? lim : left;
+                lim = lim < 6 ? lim : 6;
+                const uint32_t w = (0u - gl * (fl * (2u - fl * fl))) & ((1u << lim) - 1u);
+                gl += fl * w;
+                q += u * (int32_t)w;
+                r += v * (int32_t)w;
             }
             L30 nf, ng, nd, ne;
             l30_row(nf, f, g, u, v, 0, m);

@@ -19,6 +19,7 @@
 
 #include "hs_curve.cuh"
 #include "hs_internal.h"
+#include "hs_quad.cuh"
 
 namespace hs {
 
@@ -370,36 +371,6 @@ __global__ void __launch_bounds__(128) k_accumulate_level(const uint4 *__restric
     }
 }
 
-// Out-of-line point operations for the latency-bound level-2 reduction kernels
-// (k_window_chunks, k_window_sum): with about one warp per scheduler their
-// inlined copies overflow the instruction cache, while one shared body stays
-// resident (a call costs a few dozen instructions next to the ~2000 of an
-// addition).  The points cross the call by value.  A form that passed them by
-// address (the caller's local memory, result stored after both operands were
-// read) gave wrong sums on this toolchain for sm_103a, in every MSM, while
-// this form has passed every parity test; the l2_add / l2_dbl wrappers keep
-// the call sites in the by-address shape.
-template <class C>
-__device__ __noinline__ Xyzz l2_addv(const Xyzz a, const Xyzz b)
-{
-    return Group<C>::add(a, b);
-}
-template <class C>
-__device__ __noinline__ Xyzz l2_dblv(const Xyzz a)
-{
-    return Group<C>::dbl(a);
-}
-template <class C>
-__device__ __forceinline__ void l2_add(Xyzz *r, const Xyzz *a, const Xyzz *b)
-{
-    *r = l2_addv<C>(*a, *b);
-}
-template <class C>
-__device__ __forceinline__ void l2_dbl(Xyzz *r, const Xyzz *a)
-{
-    *r = l2_dblv<C>(*a);
-}
-
 // ---------------------------------------------------------------------------
 // 3. folding buckets that were cut into several segments
 // ---------------------------------------------------------------------------
@@ -506,180 +477,146 @@ __global__ void __launch_bounds__(128, 4) k_reduce_groups(const uint32_t *__rest
 // and the window sum is S = sum_b C_b + m0 RED_CHUNK sum_b b R_b.  Each step
 // is a short running sum, a log-depth scan or tree, and log2 of a power of two
 // doublings: no scalar multiples by group index.
-// Shared-memory points are stored word-group-major (uint4 c of thread i at
-// c * N + i), so a warp's 16-byte accesses to one uint4 of consecutive threads
-// fall in distinct banks.
-__device__ __forceinline__ void st_fe_soa(uint4 *sh, uint32_t c, uint32_t i, uint32_t N, const Fe &f)
-{
-    sh[(2 * c) * N + i] = make_uint4(f.w[0], f.w[1], f.w[2], f.w[3]);
-    sh[(2 * c + 1) * N + i] = make_uint4(f.w[4], f.w[5], f.w[6], f.w[7]);
-}
+// Both kernels work on quads (hs_quad.cuh): with one thread per point, an
+// addition's 14 products in sequence set their time (113 + 71 us on F_p and 171 +
+// 115 us on F_q for one MSM of 2^20 points).
 
-__device__ __forceinline__ Fe ld_fe_soa(const uint4 *sh, uint32_t c, uint32_t i, uint32_t N)
-{
-    const uint4 a = sh[(2 * c) * N + i], b = sh[(2 * c + 1) * N + i];
-    Fe f;
-    f.w[0] = a.x; f.w[1] = a.y; f.w[2] = a.z; f.w[3] = a.w;
-    f.w[4] = b.x; f.w[5] = b.y; f.w[6] = b.z; f.w[7] = b.w;
-    return f;
-}
-
-__device__ __forceinline__ void st_soa(uint4 *sh, uint32_t i, uint32_t N, const Xyzz &p)
-{
-    st_fe_soa(sh, 0, i, N, p.X);
-    st_fe_soa(sh, 1, i, N, p.Y);
-    st_fe_soa(sh, 2, i, N, p.ZZ);
-    st_fe_soa(sh, 3, i, N, p.ZZZ);
-}
-
-__device__ __forceinline__ Xyzz ld_soa(const uint4 *sh, uint32_t i, uint32_t N)
-{
-    Xyzz p;
-    p.X = ld_fe_soa(sh, 0, i, N);
-    p.Y = ld_fe_soa(sh, 1, i, N);
-    p.ZZ = ld_fe_soa(sh, 2, i, N);
-    p.ZZZ = ld_fe_soa(sh, 3, i, N);
-    return p;
-}
-
-// inclusive suffix scan of r over the first nt threads (sh holds N points)
+// inclusive suffix scan over the first nt quads of the block (sh: one point per
+// quad); quad g holds r and returns sum_{h >= g} r_h
 template <class C>
-__device__ __forceinline__ Xyzz block_suffix_scan(uint4 *sh, uint32_t N, Xyzz r, uint32_t i, uint32_t nt)
+__device__ __forceinline__ Fe block_suffix_scan(const Quad<C> &op, uint4 *sh, Fe r, uint32_t g, uint32_t nt)
 {
-    using G = Group<C>;
-    st_soa(sh, i, N, r);
+    using Q = Quad<C>;
+    Q::store(sh, g, op.j, r);
     __syncthreads();
     for (uint32_t dl = 1; dl < nt; dl <<= 1) {
-        Xyzz o = G::inf();
-        const bool take = i + dl < nt;
-        if (take)
-            o = ld_soa(sh, i + dl, N);
+        const bool take = g + dl < nt;
+        const Fe o = take ? Q::load(sh, g + dl, op.j) : C::F::zero();
         __syncthreads();
-        if (take) {
-            l2_add<C>(&r, &r, &o);
-            st_soa(sh, i, N, r);
+        if (__any_sync(Q::ALL, take)) {
+            r = op.template add<false>(r, o, take);
+            Q::store(sh, g, op.j, r);
         }
         __syncthreads();
     }
     return r;
 }
 
-// sum of v over the first nt (a power of two) threads, result at index 0
+// sum of v over the first nt (a power of two) quads; quad 0 returns it
 template <class C>
-__device__ __forceinline__ void block_tree_sum(uint4 *sh, uint32_t N, const Xyzz &v, uint32_t i, uint32_t nt)
+__device__ __forceinline__ Fe block_tree_sum(const Quad<C> &op, uint4 *sh, Fe v, uint32_t g, uint32_t nt)
 {
-    using G = Group<C>;
-    __syncthreads();
-    st_soa(sh, i, N, v);
+    using Q = Quad<C>;
+    Q::store(sh, g, op.j, v);
     __syncthreads();
     for (uint32_t stride = nt / 2; stride > 0; stride >>= 1) {
-        if (i < stride) {
-            Xyzz x = ld_soa(sh, i, N), y = ld_soa(sh, i + stride, N);
-            l2_add<C>(&x, &x, &y);
-            st_soa(sh, i, N, x);
+        if ((g & ~7u) < stride) {  // whole warps
+            const bool take = g < stride;
+            const Fe o = take ? Q::load(sh, g + stride, op.j) : C::F::zero();
+            v = op.template add<false>(v, o, take);
         }
         __syncthreads();
+        if (g < stride)
+            Q::store(sh, g, op.j, v);
+        __syncthreads();
     }
+    return v;
 }
 
-// k_window_chunks: thread i of a chunk first runs a top-down running sum over
-// its q consecutive groups (lo = t0 + i q):
-//     r_i = sum run_t,  w_i = sum (t - lo) run_t,  a_i = sum acc_t,
-// then the block scans r (X_i = sum_{j >= i} r_j) and thread i contributes
-//     a_i + m0 (w_i + q X_i [i >= 1]),
-// which sums to C_b; X_0 is R_b.  q = 4 groups per thread keeps both the
+// One step of level 2 on a block: over the nt pairs (acc_t, run_t) at in[lo0 ..],
+//     sum_t acc_t + mult sum_t t run_t   (returned on quad 0; mult a power of two),
+// and sum_t run_t (quad 0's r).  Quad g first runs a top-down running sum over
+// its q consecutive pairs (first one t = g q):
+//     r_g = sum run_t,  w_g = sum (t - g q) run_t,  a_g = sum acc_t,
+// then the block scans r (X_g = sum_{h >= g} r_h) and quad g contributes
+//     a_g + mult (w_g + q X_g [g >= 1]).
+template <class C>
+__device__ __forceinline__ Fe weighted_sum(const Quad<C> &op, uint4 *sh, const uint4 *__restrict__ in, size_t lo0,
+                                           uint32_t nt, uint32_t q, uint32_t mult, Fe &r)
+{
+    using F = typename C::F;
+    using Q = Quad<C>;
+    const uint32_t g = threadIdx.x >> 2, P = nt / q;
+    const bool warp_in = (g & ~7u) < P, in_p = g < P;
+    Fe a = F::zero(), w = F::zero();
+    r = F::zero();
+    if (warp_in) {
+        const size_t lo = lo0 + (size_t)g * q;
+        for (int u = (int)q - 1; u >= 0; u--) {
+            const Fe ta = in_p ? Q::load(in, 2 * (lo + u), op.j) : F::zero();
+            const Fe tr = in_p ? Q::load(in, 2 * (lo + u) + 1, op.j) : F::zero();
+            a = op.template add<false>(a, ta, in_p);
+            r = op.template add<false>(r, tr, in_p);
+            if (u > 0)
+                w = op.template add<false>(w, r, in_p);
+        }
+    }
+    r = block_suffix_scan<C>(op, sh, r, g, P);
+    Fe v = F::zero();
+    if (warp_in) {
+        v = g >= 1 ? r : F::zero();
+        for (uint32_t m = q; m > 1; m >>= 1)
+            v = op.dbl(v);
+        v = op.template add<false>(v, w, true);
+        for (uint32_t m = mult; m > 1; m >>= 1)
+            v = op.dbl(v);
+        v = op.template add<false>(v, a, true);
+    }
+    return block_tree_sum<C>(op, sh, v, g, P);
+}
+
+// quads of a level-2 block, and groups per quad: RED_CHUNK_Q keeps both the
 // sequential part and the scans' extra work small; in a plan of few windows
-// (latency-bound) a window of at most 64 groups takes one per thread, so that
-// only the scan is serial.
+// (wide: latency-bound) as few as fill the block, so that only the scan is serial
 constexpr uint32_t RED_CHUNK_Q = 4;
-constexpr uint32_t RED_CHUNK_THREADS = RED_CHUNK / RED_CHUNK_Q;
+constexpr uint32_t RED_QUADS = RED_CHUNK / RED_CHUNK_Q;
 
 // DIRECT: every window of the batch is one chunk (T <= RED_CHUNK), so C_b is
 // already the window sum and goes straight to S (k_window_sum is skipped).
 template <class C, bool DIRECT>
-__global__ void __launch_bounds__(RED_CHUNK_THREADS) k_window_chunks(const uint4 *__restrict__ in,
-                                                                    const MsmDesc *__restrict__ desc, uint32_t M,
-                                                                    uint4 *__restrict__ outC, int wide)
+__global__ void __launch_bounds__(RED_QUADS * 4) k_window_chunks(const uint4 *__restrict__ in,
+                                                                const MsmDesc *__restrict__ desc, uint32_t M,
+                                                                uint4 *__restrict__ outC, int wide)
 {
-    using G = Group<C>;
-    __shared__ uint4 sh[RED_CHUNK_THREADS * 8], sa[RED_CHUNK_THREADS * 8];
-    const uint32_t ch = blockIdx.x, i = threadIdx.x;
+    using Q = Quad<C>;
+    __shared__ uint4 sh[RED_QUADS * 8];
+    const Q op(threadIdx.x);
+    const uint32_t ch = blockIdx.x;
     const uint32_t mi = find_msm(M, ch, [&](uint32_t k) { return desc[k].chunk_base; });
     const MsmDesc d = desc[mi];
     const uint32_t nbk = d.T > RED_CHUNK ? d.T / RED_CHUNK : 1;
     const uint32_t nt = d.T < RED_CHUNK ? d.T : RED_CHUNK;
-    // groups per thread: RED_CHUNK_Q, or (wide: a plan of few windows, so
-    // latency-bound) as few as fill the block, the scan taking the rest
-    const uint32_t q = wide ? (nt > RED_CHUNK_THREADS ? nt / RED_CHUNK_THREADS : 1)
-                            : (nt < RED_CHUNK_Q ? nt : RED_CHUNK_Q);
-    const uint32_t P = nt / q;
+    const uint32_t q = wide ? (nt > RED_QUADS ? nt / RED_QUADS : 1) : (nt < RED_CHUNK_Q ? nt : RED_CHUNK_Q);
     const uint32_t local = ch - d.chunk_base;
     const uint32_t k = local / nbk, b = local % nbk;
-    Xyzz r = G::inf(), w = G::inf();
-    if (i < P) {
-        const size_t lo = (size_t)d.group_base + (size_t)k * d.T + (size_t)b * RED_CHUNK + (size_t)i * q;
-        // a_i waits in shared memory: with it, r and w in registers across the
-        // calls the kernel spills
-        Xyzz a = G::inf();
-        for (int u = (int)q - 1; u >= 0; u--) {
-            const Xyzz t = load_xyzz(in + 16 * (lo + u));
-            l2_add<C>(&a, &a, &t);
-        }
-        st_soa(sa, i, RED_CHUNK_THREADS, a);
-        for (int u = (int)q - 1; u >= 0; u--) {
-            const Xyzz t = load_xyzz(in + 16 * (lo + u) + 8);
-            l2_add<C>(&r, &r, &t);
-            if (u > 0)
-                l2_add<C>(&w, &w, &r);
-        }
-    }
-    r = block_suffix_scan<C>(sh, RED_CHUNK_THREADS, r, i, P);
-    Xyzz v = (i >= 1 && i < P) ? r : G::inf();
-    for (uint32_t m = q; m > 1; m >>= 1)
-        l2_dbl<C>(&v, &v);
-    l2_add<C>(&v, &v, &w);
-    for (uint32_t m = d.m0; m > 1; m >>= 1)
-        l2_dbl<C>(&v, &v);
-    if (i < P) {
-        const Xyzz a = ld_soa(sa, i, RED_CHUNK_THREADS);
-        l2_add<C>(&v, &v, &a);
-    }
-    block_tree_sum<C>(sh, RED_CHUNK_THREADS, v, i, P);
-    if (i == 0) {
-        if (DIRECT) {
-            store_xyzz(outC + 8 * (size_t)ch, ld_soa(sh, 0, RED_CHUNK_THREADS));
-        } else {
-            store_xyzz(outC + 16 * (size_t)ch, ld_soa(sh, 0, RED_CHUNK_THREADS));
-            store_xyzz(outC + 16 * (size_t)ch + 8, r);  // thread 0's suffix sum is the chunk's run total
-        }
+    Fe r;
+    const Fe v = weighted_sum<C>(op, sh, in, (size_t)d.group_base + (size_t)k * d.T + (size_t)b * RED_CHUNK, nt, q,
+                                 d.m0, r);
+    if (threadIdx.x < 4) {
+        Q::store(outC, DIRECT ? (size_t)ch : 2 * (size_t)ch, op.j, v);
+        if (!DIRECT)
+            Q::store(outC, 2 * (size_t)ch + 1, op.j, r);  // quad 0's suffix sum is the chunk's run total
     }
 }
 
 template <class C>
-__global__ void __launch_bounds__(RED_CHUNK) k_window_sum(const uint4 *__restrict__ inC,
-                                                         const MsmDesc *__restrict__ desc, uint32_t M,
-                                                         uint4 *__restrict__ S)
+__global__ void __launch_bounds__(RED_QUADS * 4) k_window_sum(const uint4 *__restrict__ inC,
+                                                             const MsmDesc *__restrict__ desc, uint32_t M,
+                                                             uint4 *__restrict__ S)
 {
-    using G = Group<C>;
-    __shared__ uint4 sh[RED_CHUNK * 8];
-    const uint32_t s = blockIdx.x, i = threadIdx.x;
+    using Q = Quad<C>;
+    __shared__ uint4 sh[RED_QUADS * 8];
+    const Q op(threadIdx.x);
+    const uint32_t s = blockIdx.x;
     const uint32_t mi = find_msm(M, s, [&](uint32_t k) { return desc[k].win_base; });
     const MsmDesc d = desc[mi];
     const uint32_t nbk = d.T > RED_CHUNK ? d.T / RED_CHUNK : 1;
-    Xyzz cb = G::inf(), r = G::inf();
-    if (i < nbk) {
-        const size_t c = (size_t)d.chunk_base + (size_t)(s - d.win_base) * nbk + i;
-        cb = load_xyzz(inC + 16 * c);
-        r = load_xyzz(inC + 16 * c + 8);
-    }
-    r = block_suffix_scan<C>(sh, RED_CHUNK, r, i, nbk);
-    Xyzz v = (i >= 1 && i < nbk) ? r : G::inf();
-    for (uint32_t m = d.m0 * RED_CHUNK; m > 1 && nbk > 1; m >>= 1)
-        l2_dbl<C>(&v, &v);
-    l2_add<C>(&v, &v, &cb);
-    block_tree_sum<C>(sh, RED_CHUNK, v, i, nbk);
-    if (i == 0)
-        store_xyzz(S + 8 * (size_t)s, ld_soa(sh, 0, RED_CHUNK));
+    const uint32_t q = nbk > RED_QUADS ? nbk / RED_QUADS : 1;
+    Fe r;
+    const Fe v = weighted_sum<C>(op, sh, inC, (size_t)d.chunk_base + (size_t)(s - d.win_base) * nbk, nbk, q,
+                                 d.m0 * RED_CHUNK, r);
+    if (threadIdx.x < 4)
+        Q::store(S, s, op.j, v);
 }
 
 // ---------------------------------------------------------------------------
@@ -1088,391 +1025,171 @@ __global__ void __launch_bounds__(128, 1) k_combine(const uint4 *__restrict__ S,
     }
 }
 
-// Point operations on groups of eight lanes (four groups per warp): the
-// independent products of a formula stage run on different lanes of the group,
-// each in eight 32-bit limbs, so an addition is 4 product stages and a
-// doubling 3, against 14 and 9 products in sequence on one thread; the linear
-// steps are done by the group's lane 0.  Each group keeps its points and
-// temporaries in its own shared slot file and synchronises only its own lanes,
-// so groups may take different branches.  The formulas are Group's (add-2008-s,
-// dbl-2008-s-1 with a = -3), complete.
-enum GroupSlot : int {
-    GRUN = 0, GACC = 4, GTMP = 8,  // points: X, Y, ZZ, ZZZ at base + 0..3
-    GU = 12, GV, GW, GS, GM, GM2, GT, GA, GB, GD, GYA, GYB, GXN, GZZN, GZZZN,
-    GU1, GU2, GS1, GS2, GZ12, GZZZ12, GP, GR, GPP, GRR, GPPP, GQ,
-    GNSLOTS
-};
-
-struct GroupSlots {
-    Fe f[GNSLOTS];
-    int flag;
-};
-
-template <class C>
-struct Group8 {
-    using F = typename C::F;
-    GroupSlots *sf;
-    int gl;          // lane within the group
-    unsigned gmask;  // the group's lanes in the warp
-
-    __device__ __forceinline__ void sync() const { __syncwarp(gmask); }
-
-    // slot lists packed six bits per lane: lane k's slot is bits 6k..6k+5
-    __device__ __forceinline__ static constexpr uint64_t pk(int s0, int s1 = 0, int s2 = 0, int s3 = 0, int s4 = 0,
-                                                           int s5 = 0)
-    {
-        return (uint64_t)s0 | (uint64_t)s1 << 6 | (uint64_t)s2 << 12 | (uint64_t)s3 << 18 | (uint64_t)s4 << 24 |
-               (uint64_t)s5 << 30;
-    }
-
-    // lanes gl < width: f[d[gl]] = f[a[gl]] * f[b[gl]]
-    __device__ __forceinline__ void products(int width, uint64_t a, uint64_t b, uint64_t d) const
-    {
-        sync();
-        if (gl < width) {
-            const int sh = 6 * gl;
-            const Fe x = sf->f[(a >> sh) & 63], y = sf->f[(b >> sh) & 63];
-            sf->f[(d >> sh) & 63] = F::mul(x, y);
-        }
-        sync();
-    }
-
-    __device__ __forceinline__ bool is_inf(int base) const { return F::is_exact_zero(sf->f[base + 2]); }
-
-    __device__ __forceinline__ void set_inf(int base) const
-    {
-        sync();
-        if (gl < 4)
-            sf->f[base + gl] = F::zero();
-        sync();
-    }
-
-    __device__ __forceinline__ void copy(int dst, int src) const
-    {
-        sync();
-        if (gl < 4)
-            sf->f[dst + gl] = sf->f[src + gl];
-        sync();
-    }
-
-    // p = 2p (p at base)
-    __device__ void dbl(int base) const
-    {
-        sync();
-        if (is_inf(base))
-            return;
-        const int X = base, Y = base + 1, ZZ = base + 2, ZZZ = base + 3;
-        if (gl == 0) {
-            sf->f[GU] = F::dbl(sf->f[Y]);
-            sf->f[GA] = F::sub(sf->f[X], sf->f[ZZ]);
-            sf->f[GB] = F::add(sf->f[X], sf->f[ZZ]);
-        }
-        products(2, pk(GU, GA), pk(GU, GB), pk(GV, GT));  // V = U^2, T = (X - ZZ)(X + ZZ)
-        if (gl == 0) {
-            const Fe t = sf->f[GT];
-            sf->f[GM] = F::add(F::dbl(t), t);  // M = 3(X^2 - ZZ^2), a = -3
-        }
-        // W = U V, S = X V, M^2, ZZ' = V ZZ
-        products(4, pk(GU, X, GM, GV), pk(GV, GV, GM, ZZ), pk(GW, GS, GM2, GZZN));
-        if (gl == 0) {
-            const Fe xn = F::sub(sf->f[GM2], F::dbl(sf->f[GS]));
-            sf->f[GXN] = xn;
-            sf->f[GD] = F::sub(sf->f[GS], xn);
-        }
-        products(3, pk(GM, GW, GW), pk(GD, ZZZ, Y), pk(GYA, GZZZN, GYB));  // M (S - X'), W ZZZ, W Y
-        if (gl == 0) {
-            sf->f[X] = sf->f[GXN];
-            sf->f[Y] = F::sub(sf->f[GYA], sf->f[GYB]);
-            sf->f[ZZ] = sf->f[GZZN];
-            sf->f[ZZZ] = sf->f[GZZZN];
-            if (F::is_zero(sf->f[ZZ]))  // y = 0: no such point on a prime-order curve, kept complete
-                sf->f[X] = sf->f[Y] = sf->f[ZZ] = sf->f[ZZZ] = F::zero();
-        }
-        sync();
-    }
-
-    // p += q (p at dst, q at src)
-    __device__ void add(int dst, int src) const
-    {
-        sync();
-        if (is_inf(src))
-            return;
-        if (is_inf(dst)) {
-            copy(dst, src);
-            return;
-        }
-        const int X1 = dst, Y1 = dst + 1, ZZ1 = dst + 2, ZZZ1 = dst + 3;
-        const int X2 = src, Y2 = src + 1, ZZ2 = src + 2, ZZZ2 = src + 3;
-        products(6, pk(X1, X2, Y1, Y2, ZZ1, ZZZ1), pk(ZZ2, ZZ1, ZZZ2, ZZZ1, ZZ2, ZZZ2),
-                 pk(GU1, GU2, GS1, GS2, GZ12, GZZZ12));
-        if (gl == 0) {
-            sf->f[GP] = F::sub(sf->f[GU2], sf->f[GU1]);
-            sf->f[GR] = F::sub(sf->f[GS2], sf->f[GS1]);
-            sf->flag = F::is_zero(sf->f[GP]) ? (F::is_zero(sf->f[GR]) ? 1 : 2) : 0;
-        }
-        sync();
-        const int flag = sf->flag;
-        if (flag == 1) {  // equal points: double
-            dbl(dst);
-            return;
-        }
-        if (flag == 2) {  // opposite points
-            set_inf(dst);
-            return;
-        }
-        products(2, pk(GP, GR), pk(GP, GR), pk(GPP, GRR));
-        products(3, pk(GP, GU1, GZ12), pk(GPP, GPP, GPP), pk(GPPP, GQ, GZZN));
-        if (gl == 0) {
-            const Fe xn = F::sub(F::sub(sf->f[GRR], sf->f[GPPP]), F::dbl(sf->f[GQ]));
-            sf->f[GXN] = xn;
-            sf->f[GD] = F::sub(sf->f[GQ], xn);
-        }
-        products(3, pk(GR, GS1, GZZZ12), pk(GD, GPPP, GPPP), pk(GYA, GYB, GZZZN));
-        if (gl == 0) {
-            sf->f[X1] = sf->f[GXN];
-            sf->f[Y1] = F::sub(sf->f[GYA], sf->f[GYB]);
-            sf->f[ZZ1] = sf->f[GZZN];
-            sf->f[ZZZ1] = sf->f[GZZZN];
-        }
-        sync();
-    }
-
-    // p = 2 (x, y) for the affine point at src (x, y at src, src + 1), into dst
-    // (mdbl-2008-s-1, M = 3 x^2 - 3)
-    __device__ void dbl_affine(int dst, int src) const
-    {
-        sync();
-        if (gl == 0)
-            sf->f[GU] = F::dbl(sf->f[src + 1]);
-        products(2, pk(GU, src), pk(GU, src), pk(GV, GT));  // V = U^2, x^2
-        if (gl == 0) {
-            const Fe t = F::sub(sf->f[GT], F::one());
-            sf->f[GM] = F::add(F::dbl(t), t);
-        }
-        products(3, pk(GU, src, GM), pk(GV, GV, GM), pk(GW, GS, GM2));  // W = U V, S = x V, M^2
-        if (gl == 0) {
-            const Fe xn = F::sub(sf->f[GM2], F::dbl(sf->f[GS]));
-            sf->f[GXN] = xn;
-            sf->f[GD] = F::sub(sf->f[GS], xn);
-        }
-        products(2, pk(GM, GW), pk(GD, src + 1), pk(GYA, GYB));  // M (S - X'), W y
-        if (gl == 0) {
-            if (F::is_zero(sf->f[GV])) {  // y = 0: no such point on a prime-order curve, kept complete
-                sf->f[dst] = sf->f[dst + 1] = sf->f[dst + 2] = sf->f[dst + 3] = F::zero();
-            } else {
-                sf->f[dst] = sf->f[GXN];
-                sf->f[dst + 1] = F::sub(sf->f[GYA], sf->f[GYB]);
-                sf->f[dst + 2] = sf->f[GV];
-                sf->f[dst + 3] = sf->f[GW];
-            }
-        }
-        sync();
-    }
-
-    // p += (x, y), the affine point at src (never the identity): madd-2008-s
-    __device__ void madd(int dst, int src) const
-    {
-        sync();
-        if (is_inf(dst)) {
-            if (gl < 4)
-                sf->f[dst + gl] = gl < 2 ? sf->f[src + gl] : F::one();
-            sync();
-            return;
-        }
-        const int X1 = dst, Y1 = dst + 1, ZZ1 = dst + 2, ZZZ1 = dst + 3;
-        products(2, pk(src, src + 1), pk(ZZ1, ZZZ1), pk(GU2, GS2));  // U2 = x ZZ1, S2 = y ZZZ1
-        if (gl == 0) {
-            sf->f[GP] = F::sub(sf->f[GU2], sf->f[X1]);
-            sf->f[GR] = F::sub(sf->f[GS2], sf->f[Y1]);
-            sf->flag = F::is_zero(sf->f[GP]) ? (F::is_zero(sf->f[GR]) ? 1 : 2) : 0;
-        }
-        sync();
-        const int flag = sf->flag;
-        if (flag == 1) {  // same point: double
-            dbl_affine(dst, src);
-            return;
-        }
-        if (flag == 2) {  // opposite points
-            set_inf(dst);
-            return;
-        }
-        products(2, pk(GP, GR), pk(GP, GR), pk(GPP, GRR));
-        products(3, pk(GP, X1, ZZ1), pk(GPP, GPP, GPP), pk(GPPP, GQ, GZZN));  // PPP, Q = X1 PP, ZZ1 PP
-        if (gl == 0) {
-            const Fe xn = F::sub(F::sub(sf->f[GRR], sf->f[GPPP]), F::dbl(sf->f[GQ]));
-            sf->f[GXN] = xn;
-            sf->f[GD] = F::sub(sf->f[GQ], xn);
-        }
-        products(3, pk(GR, Y1, ZZZ1), pk(GD, GPPP, GPPP), pk(GYA, GYB, GZZZN));  // R (Q - X'), Y1 PPP, ZZZ1 PPP
-        if (gl == 0) {
-            sf->f[X1] = sf->f[GXN];
-            sf->f[Y1] = F::sub(sf->f[GYA], sf->f[GYB]);
-            sf->f[ZZ1] = sf->f[GZZN];
-            sf->f[ZZZ1] = sf->f[GZZZN];
-        }
-        sync();
-    }
-};
-
-// Window sums of a plan of few windows of at most WG_MAX_B buckets, where the
-// two-level reduction's chains of one-thread additions set the time: one block
-// of WG_GROUPS eight-lane groups per window, group g taking the q = B / groups
-// buckets [g q, (g + 1) q):
+// Window sums of a plan of few windows of at most WQ_MAX_B buckets, where the
+// two-level reduction's chains of additions set the time: one block of WQ_QUADS
+// four-lane quads per window, quad g taking the q = B / quads buckets
+// [g q, (g + 1) q):
 //     run_g = sum_j B_j,   acc_g = sum_j (j - g q + 1) B_j   (top-down running sum),
 // then S = sum_g acc_g + q sum_{g >= 1} R_g with R_g = sum_{h >= g} run_h (a
-// suffix scan over the groups), q R_g by doublings, and a tree sum.
-constexpr int WG_GROUPS = 32;
-constexpr uint32_t WG_MAX_B = 256;
+// suffix scan over the quads), q R_g by doublings, and a tree sum.  Additions
+// that no quad of a warp needs (empty buckets, identities) are skipped.
+constexpr int WQ_QUADS = 64;
+constexpr uint32_t WQ_MAX_B = 256;
 
 template <class C>
-__global__ void __launch_bounds__(WG_GROUPS * 8) k_window_groups(const uint32_t *__restrict__ seg_off,
-                                                                const uint4 *__restrict__ seg_sum,
-                                                                const MsmDesc *__restrict__ desc, uint32_t M,
-                                                                uint4 *__restrict__ S)
+__global__ void __launch_bounds__(WQ_QUADS * 4) k_window_quads(const uint32_t *__restrict__ seg_off,
+                                                              const uint4 *__restrict__ seg_sum,
+                                                              const MsmDesc *__restrict__ desc, uint32_t M,
+                                                              uint4 *__restrict__ S)
 {
-    __shared__ GroupSlots sl[WG_GROUPS];
+    using F = typename C::F;
+    using Q = Quad<C>;
+    __shared__ uint4 sh[WQ_QUADS * 8];
     const uint32_t s = blockIdx.x;
     const uint32_t mi = find_msm(M, s, [&](uint32_t k) { return desc[k].win_base; });
     const MsmDesc d = desc[mi];
     const uint32_t k = s - d.win_base;
-    const uint32_t g = threadIdx.x >> 3;
-    Group8<C> op;
-    op.sf = &sl[g];
-    op.gl = (int)(threadIdx.x & 7);
-    op.gmask = 0xffu << (8 * (g & 3));
-    const uint32_t nga = d.B < (uint32_t)WG_GROUPS ? d.B : (uint32_t)WG_GROUPS;  // B is a power of two
+    const uint32_t g = threadIdx.x >> 2;
+    const Q op(threadIdx.x);
+    const uint32_t nga = d.B < (uint32_t)WQ_QUADS ? d.B : (uint32_t)WQ_QUADS;  // B is a power of two
     const uint32_t q = d.B / nga;
     const bool active = g < nga;
-    op.set_inf(GRUN);
-    op.set_inf(GACC);
-    if (active) {
-        for (int j = (int)((g + 1) * q) - 1; j >= (int)(g * q); j--) {
-            const uint32_t kb = d.bucket_base + k * d.B + (uint32_t)j;
+    Fe run = F::zero(), acc = F::zero();
+    for (int u = (int)q - 1; u >= 0; u--) {
+        Fe t = F::zero();
+        bool take = false;
+        if (active) {
+            const uint32_t kb = d.bucket_base + k * d.B + g * q + (uint32_t)u;
             const uint32_t s0 = seg_off[kb];
-            if (seg_off[kb + 1] != s0) {
-                op.sync();
-                if (op.gl < 4)
-                    op.sf->f[GTMP + op.gl] = load_fe(seg_sum + 8 * (size_t)s0 + 2 * op.gl);
-                op.add(GRUN, GTMP);
-            }
-            op.add(GACC, GRUN);
+            take = seg_off[kb + 1] != s0;
+            if (take)
+                t = Q::load(seg_sum, s0, op.j);
         }
+        if (__any_sync(Q::ALL, take))
+            run = op.template add<false>(run, t, take);
+        const bool more = !Q::is_inf(run);
+        if (__any_sync(Q::ALL, more))
+            acc = op.template add<false>(acc, run, more);
     }
+    Q::store(sh, g, op.j, run);
     __syncthreads();
     for (uint32_t dl = 1; dl < nga; dl <<= 1) {  // R_g
-        const bool take = active && g + dl < nga;
-        if (take && op.gl < 4)
-            op.sf->f[GTMP + op.gl] = sl[g + dl].f[GRUN + op.gl];
+        bool take = g + dl < nga;
+        const Fe o = take ? Q::load(sh, g + dl, op.j) : F::zero();
+        const bool o_inf = Q::is_inf(o);
+        take = take && !o_inf;
         __syncthreads();
-        if (take)
-            op.add(GRUN, GTMP);
-        __syncthreads();
-    }
-    if (active) {  // v_g = q R_g [g >= 1] + acc_g, in GRUN
-        if (g >= 1) {
-            for (uint32_t m = q; m > 1; m >>= 1)
-                op.dbl(GRUN);
-        } else {
-            op.set_inf(GRUN);
+        if (__any_sync(Q::ALL, take)) {
+            run = op.template add<false>(run, o, take);
+            Q::store(sh, g, op.j, run);
         }
-        op.add(GRUN, GACC);
+        __syncthreads();
     }
+    // v_g = q R_g [g >= 1] + acc_g
+    Fe v = g >= 1 ? run : F::zero();
+    for (uint32_t m = q; m > 1; m >>= 1)
+        v = op.dbl(v);
+    v = op.template add<false>(v, acc, true);
+    Q::store(sh, g, op.j, v);
     __syncthreads();
     for (uint32_t st = nga / 2; st > 0; st >>= 1) {
-        if (g < st) {
-            if (op.gl < 4)
-                op.sf->f[GTMP + op.gl] = sl[g + st].f[GRUN + op.gl];
-            op.add(GRUN, GTMP);
+        if ((threadIdx.x >> 5) * 8 < st) {  // whole warps
+            const bool take = g < st;
+            const Fe o = take ? Q::load(sh, g + st, op.j) : F::zero();
+            v = op.template add<false>(v, o, take);
         }
         __syncthreads();
+        if (g < st)
+            Q::store(sh, g, op.j, v);
+        __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        Xyzz t;
-        t.X = sl[0].f[GRUN];
-        t.Y = sl[0].f[GRUN + 1];
-        t.ZZ = sl[0].f[GRUN + 2];
-        t.ZZZ = sl[0].f[GRUN + 3];
-        store_xyzz(S + 8 * (size_t)s, t);
-    }
+    if (g == 0)
+        Q::store(S, s, op.j, v);
 }
 
-// Bucket accumulation and merges of small plans on eight-lane groups (a mixed
-// addition is 4 product stages against 10 products on one thread): one group
-// per segment, then one group per bucket of 2..8 segments (more go to the
-// heavy-bucket list as in k_merge_light).  About 3.7 times the instructions
-// per entry of the one-thread form, so only for plans of at most
-// ACC_GROUPS_MAX_ENTRIES entries.
-constexpr uint64_t ACC_GROUPS_MAX_ENTRIES = 98304;
+// Bucket accumulation and merges of small plans on quads (a mixed addition is
+// 4 product stages against 10 products on one thread): one quad per segment,
+// then one quad per bucket of 2..8 segments (more go to the heavy-bucket list as
+// in k_merge_light).  16 product slots per entry against 10, so only for plans
+// of at most ACC_QUADS_MAX_ENTRIES entries.
+constexpr uint64_t ACC_QUADS_MAX_ENTRIES = 98304;
 
 template <class C>
-__global__ void __launch_bounds__(256) k_accumulate_groups(const uint4 *__restrict__ segs,
-                                                          const uint32_t *__restrict__ seg_lo,
-                                                          const uint32_t *__restrict__ seg_hi,
-                                                          const uint32_t *__restrict__ sorted,
-                                                          const uint4 *__restrict__ pts, uint4 *__restrict__ seg_sum)
+__global__ void __launch_bounds__(128) k_accumulate_quads(const uint4 *__restrict__ segs,
+                                                         const uint32_t *__restrict__ seg_lo,
+                                                         const uint32_t *__restrict__ seg_hi,
+                                                         const uint32_t *__restrict__ sorted,
+                                                         const uint4 *__restrict__ pts, uint4 *__restrict__ seg_sum)
 {
     using F = typename C::F;
-    __shared__ GroupSlots sl[32];
-    const uint32_t g = threadIdx.x >> 3;
-    Group8<C> op;
-    op.sf = &sl[g];
-    op.gl = (int)(threadIdx.x & 7);
-    op.gmask = 0xffu << (8 * (g & 3));
+    using Q = Quad<C>;
+    const Q op(threadIdx.x);
     const uint32_t S0 = *seg_lo, S = *seg_hi;
-    for (uint32_t s = S0 + blockIdx.x * 32 + g; s < S; s += gridDim.x * 32) {
-        const uint4 d = segs[s];  // start, length, destination slot
-        op.set_inf(GRUN);
-        for (uint32_t i = 0; i < d.y; i++) {
-            const uint32_t e = __ldg(sorted + d.x + i);
-            Fe x, y;
-            load_affine(pts, e & 0x7fffffffu, x, y);
-            if (F::is_exact_zero(x) && F::is_exact_zero(y))
-                continue;  // identity base
-            op.sync();
-            if (op.gl == 0)
-                op.sf->f[GTMP] = x;
-            else if (op.gl == 1)
-                op.sf->f[GTMP + 1] = (e >> 31) ? F::neg(y) : y;
-            op.madd(GRUN, GTMP);
+    const uint32_t stride = gridDim.x * (blockDim.x >> 2);
+    // a warp's eight quads take consecutive segments and leave the loop together
+    for (uint32_t w = S0 + blockIdx.x * (blockDim.x >> 2) + (threadIdx.x >> 5) * 8; w < S; w += stride) {
+        const uint32_t s = w + ((threadIdx.x >> 2) & 7);
+        const uint4 d = s < S ? segs[s] : make_uint4(0, 0, 0, 0);  // start, length, destination slot
+        const uint32_t len = __reduce_max_sync(Q::ALL, d.y);
+        Fe acc = F::zero();
+        for (uint32_t i = 0; i < len; i++) {
+            bool take = i < d.y;
+            Fe c = F::zero();
+            uint32_t e = 0;
+            if (take) {
+                e = __ldg(sorted + d.x + i);
+                if (op.j < 2) {
+                    const uint4 *src = pts + 4 * (size_t)(e & 0x7fffffffu) + 2 * op.j;
+                    const uint4 a = __ldg(src), b = __ldg(src + 1);
+                    c = Fe{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}};
+                }
+            }
+            // an identity base contributes nothing (both flags on every lane: they are shuffles)
+            const bool z = F::is_exact_zero(c);
+            const bool zx = Q::flag(z, 0), zy = Q::flag(z, 1);
+            take = take && !(zx && zy);
+            if (op.j == 1 && (e >> 31))
+                c = F::neg(c);
+            if (__any_sync(Q::ALL, take))
+                acc = op.template add<true>(acc, c, take);
         }
-        op.sync();
-        if (op.gl < 4)
-            store_fe(seg_sum + 8 * (size_t)d.z + 2 * op.gl, op.sf->f[GRUN + op.gl]);
+        if (s < S)
+            Q::store(seg_sum, d.z, op.j, acc);
     }
 }
 
 template <class C>
-__global__ void __launch_bounds__(256) k_merge_groups(const uint32_t *__restrict__ seg_off, uint32_t NB,
-                                                     uint4 *__restrict__ seg_sum, uint32_t *__restrict__ heavy,
-                                                     uint32_t *__restrict__ heavy_n, uint32_t heavy_min)
+__global__ void __launch_bounds__(128) k_merge_quads(const uint32_t *__restrict__ seg_off, uint32_t NB,
+                                                    uint4 *__restrict__ seg_sum, uint32_t *__restrict__ heavy,
+                                                    uint32_t *__restrict__ heavy_n, uint32_t heavy_min)
 {
-    __shared__ GroupSlots sl[32];
-    const uint32_t g = threadIdx.x >> 3;
-    Group8<C> op;
-    op.sf = &sl[g];
-    op.gl = (int)(threadIdx.x & 7);
-    op.gmask = 0xffu << (8 * (g & 3));
-    for (uint32_t kb = blockIdx.x * 32 + g; kb < NB; kb += gridDim.x * 32) {
-        const uint32_t s0 = seg_off[kb], ns = seg_off[kb + 1] - s0;
-        if (ns < 2)
-            continue;
-        if (ns > heavy_min) {
-            if (op.gl == 0)
-                heavy[atomicAdd(heavy_n, 1u)] = kb;
-            continue;
+    using F = typename C::F;
+    using Q = Quad<C>;
+    const Q op(threadIdx.x);
+    const uint32_t stride = gridDim.x * (blockDim.x >> 2);
+    for (uint32_t w = blockIdx.x * (blockDim.x >> 2) + (threadIdx.x >> 5) * 8; w < NB; w += stride) {
+        const uint32_t kb = w + ((threadIdx.x >> 2) & 7);
+        uint32_t s0 = 0, ns = 0;
+        if (kb < NB) {
+            s0 = seg_off[kb];
+            ns = seg_off[kb + 1] - s0;
+            if (ns > heavy_min) {
+                if (op.j == 0)
+                    heavy[atomicAdd(heavy_n, 1u)] = kb;
+                ns = 0;
+            }
         }
-        op.sync();
-        if (op.gl < 4)
-            op.sf->f[GRUN + op.gl] = load_fe(seg_sum + 8 * (size_t)s0 + 2 * op.gl);
-        for (uint32_t j = 1; j < ns; j++) {
-            op.sync();
-            if (op.gl < 4)
-                op.sf->f[GTMP + op.gl] = load_fe(seg_sum + 8 * (size_t)(s0 + j) + 2 * op.gl);
-            op.add(GRUN, GTMP);
+        const uint32_t most = __reduce_max_sync(Q::ALL, ns);
+        if (most < 2)
+            continue;
+        Fe acc = ns > 1 ? Q::load(seg_sum, s0, op.j) : F::zero();
+        for (uint32_t i = 1; i < most; i++) {
+            const bool take = i < ns;
+            const Fe o = take ? Q::load(seg_sum, s0 + i, op.j) : F::zero();
+            acc = op.template add<false>(acc, o, take);
         }
-        op.sync();
-        if (op.gl < 4)
-            store_fe(seg_sum + 8 * (size_t)s0 + 2 * op.gl, op.sf->f[GRUN + op.gl]);
+        if (ns > 1)
+            Q::store(seg_sum, s0, op.j, acc);
     }
 }
 
@@ -1480,8 +1197,8 @@ template <class C>
 cudaError_t msm_tail(Context &ctx, const BatchPlan &p, const BatchBuffers &b)
 {
     cudaStream_t st = ctx.stream;
-    // a small plan: accumulation and merges on eight-lane groups
-    const bool small = !p.ba_rounds && !p.part_slice && p.entries_bound <= ACC_GROUPS_MAX_ENTRIES;
+    // a small plan: accumulation and merges on quads
+    const bool small = !p.ba_rounds && !p.part_slice && p.entries_bound <= ACC_QUADS_MAX_ENTRIES;
     // 2. accumulate: a grid of short blocks (up to 32 per SM, several waves), each
     //    thread taking segments at a stride of the grid.  Segments come longest
     //    first, so every block gets a like mix of long and short ones; blocks end
@@ -1544,8 +1261,8 @@ cudaError_t msm_tail(Context &ctx, const BatchPlan &p, const BatchBuffers &b)
         const size_t nh = (size_t)(p.L + 1) * p.hist_blocks;
         cudaEvent_t ev0 = nullptr;
         prof_begin(ctx, &ev0);
-        k_accumulate_groups<C><<<blocks, 256, 0, st>>>(b.segs, b.len_scan, b.len_scan + nh, b.sorted, b.points,
-                                                       b.seg_sum);
+        k_accumulate_quads<C><<<blocks, 128, 0, st>>>(b.segs, b.len_scan, b.len_scan + nh, b.sorted, b.points,
+                                                      b.seg_sum);
         HS_LAUNCH_CHECK(ctx);
         prof_end(ctx, ev0, p.entries_pinned);
     } else {
@@ -1584,7 +1301,7 @@ cudaError_t msm_tail(Context &ctx, const BatchPlan &p, const BatchBuffers &b)
         if (small) {
             const unsigned mb = (unsigned)std::max<uint32_t>(1, std::min<uint32_t>((p.NB + 31) / 32,
                                                                                    (uint32_t)ctx.sm_count * 8));
-            k_merge_groups<C><<<mb, 256, 0, st>>>(b.seg_off, p.NB, b.seg_sum, b.heavy, b.heavy_n, 8);
+            k_merge_quads<C><<<mb, 128, 0, st>>>(b.seg_off, p.NB, b.seg_sum, b.heavy, b.heavy_n, 8);
         } else {
             k_merge_light<C><<<(p.NB + threads - 1) / threads, threads, 0, st>>>(b.seg_off, p.NB, b.seg_sum,
                                                                                b.heavy, b.heavy_n, 8);
@@ -1594,10 +1311,10 @@ cudaError_t msm_tail(Context &ctx, const BatchPlan &p, const BatchBuffers &b)
         HS_LAUNCH_CHECK(ctx);
     }
     // 4. bucket reduction: group running sums, then one block per window; a
-    //    plan of few windows of at most WG_MAX_B buckets reduces each window on
-    //    one block of eight-lane groups
-    if (p.max_B <= WG_MAX_B && p.WS <= 4u * (uint32_t)ctx.sm_count) {
-        k_window_groups<C><<<p.WS, WG_GROUPS * 8, 0, st>>>(b.seg_off, b.seg_sum, b.desc, p.M, b.redS);
+    //    plan of few windows of at most WQ_MAX_B buckets reduces each window on
+    //    one block of quads
+    if (p.max_B <= WQ_MAX_B && p.WS <= 4u * (uint32_t)ctx.sm_count) {
+        k_window_quads<C><<<p.WS, WQ_QUADS * 4, 0, st>>>(b.seg_off, b.seg_sum, b.desc, p.M, b.redS);
         HS_LAUNCH_CHECK(ctx);
     } else {
         const int threads = 128;
@@ -1613,14 +1330,14 @@ cudaError_t msm_tail(Context &ctx, const BatchPlan &p, const BatchBuffers &b)
         // 64..65536 points 1.5% faster with four.)
         const int wide = p.CH <= 4u * (uint32_t)ctx.sm_count || p.max_T <= 16;
         const uint32_t t2 =
-            std::max<uint32_t>(32, std::min<uint32_t>(RED_CHUNK_THREADS, wide ? p.max_T : p.max_T / RED_CHUNK_Q));
+            std::max<uint32_t>(32, 4 * std::min<uint32_t>(RED_QUADS, wide ? p.max_T : p.max_T / RED_CHUNK_Q));
         if (p.max_nbk == 1) {  // one chunk per window: chunk index == window slot
             k_window_chunks<C, true><<<p.CH, t2, 0, st>>>(b.redA, b.desc, p.M, b.redS, wide);
             HS_LAUNCH_CHECK(ctx);
         } else {
             k_window_chunks<C, false><<<p.CH, t2, 0, st>>>(b.redA, b.desc, p.M, b.redC, wide);
             HS_LAUNCH_CHECK(ctx);
-            const uint32_t t3 = std::max<uint32_t>(32, std::min<uint32_t>(RED_CHUNK, p.max_nbk));
+            const uint32_t t3 = std::max<uint32_t>(32, 4 * std::min<uint32_t>(RED_QUADS, p.max_nbk));
             k_window_sum<C><<<p.WS, t3, 0, st>>>(b.redC, b.desc, p.M, b.redS);
             HS_LAUNCH_CHECK(ctx);
         }
