@@ -93,7 +93,7 @@ struct Context {
     //   threads: 6.06 ms per pair with one round on both, 5.91 ms without one
     //   on Helios).
     bool ba_set[2] = {false, false};
-    uint32_t fixed_ba_rounds[2] = {0, 1};
+    uint32_t fixed_ba_rounds[2] = {0, 2};
     uint32_t host_ba_rounds[2] = {0, 1};
     std::vector<GraphEntry> graphs;
     DeviceArena arena;
@@ -199,9 +199,9 @@ struct BatchPlan {
     uint32_t ba_blocks[3] = {};  // blocks of round r's kernels (BA_K * BA_BT outputs each)
 };
 
-// batch-affine rounds: outputs per thread and threads per block of a round (one
-// shared inversion per block), and the rounds at most
-constexpr uint32_t BA_PLAN_K = 16;
+// batch-affine rounds: outputs per thread and threads per block of a round, and the
+// rounds at most
+constexpr uint32_t BA_PLAN_K = 32;
 constexpr uint32_t BA_PLAN_BT = 128;
 constexpr uint32_t BA_MAX_ROUNDS = 3;
 
@@ -233,9 +233,7 @@ struct BatchBuffers {
     // [offsets[k] >> r, offsets[k+1] >> r) of its level
     uint4 *ba_lvl[2] = {};              // round outputs, affine (4 uint4 each): odd rounds [0], even [1]
     uint4 *ba_pre = nullptr;            // round-1 bound of outputs: exclusive prefix products (2 uint4 each)
-    uint4 *ba_co = nullptr;             // per thread: product of the other threads' totals of its block
-    uint4 *ba_tot = nullptr;            // per block: product of its denominators
-    uint4 *ba_inv = nullptr;            // per block: its inverse
+    uint4 *ba_tot = nullptr;            // per thread: product of its denominators, then its inverse
     // host inputs: the accumulation of part j waits for ready[j] (null: bases resident)
     cudaEvent_t ready[2] = {nullptr, nullptr};
 };

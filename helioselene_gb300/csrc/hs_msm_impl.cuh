@@ -27,14 +27,40 @@ namespace hs {
 // ---------------------------------------------------------------------------
 // memory helpers
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void load_affine(const uint4 *__restrict__ pts, uint32_t idx, Fe &x, Fe &y)
+// One field element per access: 32-byte loads and stores of global memory.  A warp's
+// gather of 64-byte points is then two requests per point instead of four, and a
+// stream of elements is full sectors.  The library's own buffers are 256-byte
+// aligned; the caller's points need only 16 bytes, so their loads take `wide`, the
+// same for a whole launch.
+__device__ __forceinline__ Fe ldg_fe(const uint4 *p)
+{
+    Fe f;
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(f.w[0]), "=r"(f.w[1]), "=r"(f.w[2]), "=r"(f.w[3]), "=r"(f.w[4]), "=r"(f.w[5]), "=r"(f.w[6]), "=r"(f.w[7])
+        : "l"(p));
+    return f;
+}
+__device__ __forceinline__ Fe ldg_fe(const uint4 *p, bool wide)
+{
+    if (wide)
+        return ldg_fe(p);
+    const uint4 a = __ldg(p), b = __ldg(p + 1);
+    return Fe{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}};
+}
+__device__ __forceinline__ bool wide_points(const uint4 *pts) { return (reinterpret_cast<uintptr_t>(pts) & 31) == 0; }
+
+__device__ __forceinline__ void stg_fe(uint4 *p, const Fe &f)
+{
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(f.w[0]), "r"(f.w[1]),
+                 "r"(f.w[2]), "r"(f.w[3]), "r"(f.w[4]), "r"(f.w[5]), "r"(f.w[6]), "r"(f.w[7])
+                 : "memory");
+}
+
+__device__ __forceinline__ void load_affine(const uint4 *__restrict__ pts, uint32_t idx, Fe &x, Fe &y, bool wide)
 {
     const uint4 *p = pts + 4 * (size_t)idx;
-    uint4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2), d = __ldg(p + 3);
-    x.w[0] = a.x; x.w[1] = a.y; x.w[2] = a.z; x.w[3] = a.w;
-    x.w[4] = b.x; x.w[5] = b.y; x.w[6] = b.z; x.w[7] = b.w;
-    y.w[0] = c.x; y.w[1] = c.y; y.w[2] = c.z; y.w[3] = c.w;
-    y.w[4] = d.x; y.w[5] = d.y; y.w[6] = d.z; y.w[7] = d.w;
+    x = ldg_fe(p, wide);
+    y = ldg_fe(p + 2, wide);
 }
 
 __device__ __forceinline__ void store_fe(uint4 *o, const Fe &f)
@@ -70,6 +96,15 @@ __device__ __forceinline__ Xyzz load_xyzz(const uint4 *o)
     return p;
 }
 
+// the library's own buffers in global memory
+__device__ __forceinline__ void stg_xyzz(uint4 *o, const Xyzz &p)
+{
+    stg_fe(o, p.X);
+    stg_fe(o + 2, p.Y);
+    stg_fe(o + 4, p.ZZ);
+    stg_fe(o + 6, p.ZZZ);
+}
+
 // ---------------------------------------------------------------------------
 // 2. bucket accumulation: one thread per segment of <= L entries (segments come
 //    longest first, so the lanes of a warp do equal work).  The launch takes the
@@ -78,7 +113,7 @@ __device__ __forceinline__ Xyzz load_xyzz(const uint4 *o)
 //    continues the sum stored in its slot by the earlier part.
 // ---------------------------------------------------------------------------
 template <class C, bool RESUME>
-__global__ void __launch_bounds__(128) k_accumulate(const uint4 *__restrict__ segs, const uint32_t *__restrict__ seg_lo,
+__global__ void __launch_bounds__(128, 4) k_accumulate(const uint4 *__restrict__ segs, const uint32_t *__restrict__ seg_lo,
                                                    const uint32_t *__restrict__ seg_hi,
                                                    const uint32_t *__restrict__ sorted, const uint4 *__restrict__ pts,
                                                    uint4 *__restrict__ seg_sum)
@@ -86,20 +121,21 @@ __global__ void __launch_bounds__(128) k_accumulate(const uint4 *__restrict__ se
     using G = Group<C>;
     using F = typename C::F;
     const uint32_t S0 = *seg_lo, S = *seg_hi;
+    const bool wide = wide_points(pts);
     for (uint32_t s = S0 + blockIdx.x * blockDim.x + threadIdx.x; s < S; s += gridDim.x * blockDim.x) {
         const uint4 d = segs[s];  // start, length, destination slot, continue
         Xyzz acc = (RESUME && d.w) ? load_xyzz(seg_sum + 8 * (size_t)d.z) : G::inf();
         for (uint32_t i = 0; i < d.y; i++) {
             const uint32_t e = __ldg(sorted + d.x + i);
             Fe x, y;
-            load_affine(pts, e & 0x7fffffffu, x, y);
+            load_affine(pts, e & 0x7fffffffu, x, y, wide);
             if (F::is_exact_zero(x) && F::is_exact_zero(y))
                 continue;  // identity base (the reference's Z == 0 input) contributes nothing
             if (e >> 31)
                 y = F::neg(y);
             G::add_affine(acc, x, y);
         }
-        store_xyzz(seg_sum + 8 * (size_t)d.z, acc);
+        stg_xyzz(seg_sum + 8 * (size_t)d.z, acc);
     }
 }
 
@@ -117,98 +153,81 @@ __global__ void __launch_bounds__(128) k_accumulate(const uint4 *__restrict__ se
 // pairs.  The divisions of a round share inversions by Montgomery's trick
 // (fp/include/fp_batch_invert.h:61-114 applied across a wave of additions):
 //   k_ba_pairs   lane l of warp tile w takes outputs w*32K + l + 32k (k < K):
-//                denominators, their running product (each output's exclusive
-//                prefix is stored), then a product tree over the block's
-//                threads; the block total goes out and each thread keeps its
-//                co-product (the product of the other threads' totals);
-//   k_ba_invert  one inversion per block total (BA_K * BA_BT additions);
-//   k_ba_finish  1/T_t = inv(block) * co-product, then each output walks back:
+//                denominators and their running product (each output's exclusive
+//                prefix and the thread's total are stored);
+//   k_ba_invert  the totals' inverses, one inversion shared by a block's BA_G *
+//                BA_INV_BT totals (so by BA_K times as many additions);
+//   k_ba_finish  each output walks back from the thread's inverse:
 //                1/d = (1/prefix through d) * (prefix before d), and the sum.
+// (A product tree over each block of k_ba_pairs, one inversion per block, held up
+// its warps at the tree's fourteen barriers: 248 + 30 us and 199 + 30 us on F_q and F_p
+// for one MSM of 2^20 points.)
 // Pairs with equal x double (d = 2 y_a) or cancel (the identity, d = 1); an
 // identity operand (affine (0,0), or a padding entry) takes d = 1 and the
 // other operand is copied.  The last round's sums are folded into XYZZ bucket
 // sums by k_accumulate_level.
 constexpr int BA_K = (int)BA_PLAN_K;    // outputs per thread
-constexpr int BA_BT = (int)BA_PLAN_BT;  // threads per block: one shared inversion per BA_K * BA_BT outputs
+constexpr int BA_BT = (int)BA_PLAN_BT;  // threads per block
 constexpr uint32_t PAD_ENTRY = 0xffffffffu;
 
 enum BaKind : int { BA_ADD, BA_DBL, BA_COPY_A, BA_COPY_B, BA_ZERO };
 
-__device__ __forceinline__ Fe ba_ld(const uint4 *p)
-{
-    const uint4 a = __ldg(p), b = __ldg(p + 1);
-    Fe f;
-    f.w[0] = a.x; f.w[1] = a.y; f.w[2] = a.z; f.w[3] = a.w;
-    f.w[4] = b.x; f.w[5] = b.y; f.w[6] = b.z; f.w[7] = b.w;
-    return f;
-}
-
-// Where item i of a round's input lives: round 1 reads entry i (point index |
-// sign << 31; PAD_ENTRY is the identity, src null), later rounds the previous
-// level's affine sum i.
-template <bool FIRST>
-__device__ __forceinline__ const uint4 *ba_src(uint32_t e, const uint4 *__restrict__ pts,
-                                              const uint4 *__restrict__ lvl, uint32_t i, bool &neg)
-{
-    if (FIRST) {
-        neg = (e >> 31) != 0;
-        return e == PAD_ENTRY ? nullptr : pts + 4 * (size_t)(e & 0x7fffffffu);
-    }
-    neg = false;
-    return lvl + 4 * (size_t)i;
-}
-
-// y of an item (negated for a negative round-1 digit; the identity left (0,0))
-template <class C>
-__device__ __forceinline__ Fe ba_load_y(const uint4 *src, bool neg, const Fe &x)
-{
+// The two items of an output.  Round 1 reads entries 2q and 2q + 1 (point index |
+// sign << 31; PAD_ENTRY is the identity), later rounds items 2q and 2q + 1 of the
+// previous level's affine sums.
+template <class C, bool FIRST>
+struct BaInput {
     using F = typename C::F;
-    const Fe y = ba_ld(src + 2);
-    return (neg && !(F::is_exact_zero(x) && F::is_exact_zero(y))) ? F::neg(y) : y;
-}
+    const uint2 *entries;
+    const uint4 *base;  // the points, or the previous level
+    bool wide;
 
-// Kind and denominator of output q (items 2q and 2q+1).  With FULL every
-// coordinate is loaded (for the sum); without, a y coordinate only when the
-// case needs it (identity check, equal x).
-template <class C, bool FIRST, bool FULL>
-__device__ __forceinline__ int ba_item(const uint32_t *__restrict__ sorted, const uint4 *__restrict__ pts,
-                                       const uint4 *__restrict__ lvl, uint32_t q, Fe &xa, Fe &ya, Fe &xb, Fe &yb,
-                                       Fe &d)
-{
-    using F = typename C::F;
-    uint32_t ea = 0, eb = 0;
-    if (FIRST) {
-        const uint2 e = __ldg(reinterpret_cast<const uint2 *>(sorted) + q);
-        ea = e.x;
-        eb = e.y;
+    __device__ __forceinline__ BaInput(const uint32_t *sorted, const uint4 *pts, const uint4 *lvl)
+        : entries(reinterpret_cast<const uint2 *>(sorted)), base(FIRST ? pts : lvl), wide(!FIRST || wide_points(pts))
+    {
     }
-    bool na, nb;
-    const uint4 *sa = ba_src<FIRST>(ea, pts, lvl, 2 * q, na);
-    const uint4 *sb = ba_src<FIRST>(eb, pts, lvl, 2 * q + 1, nb);
-    d = F::one();
-    xa = sa ? ba_ld(sa) : F::zero();
-    xb = sb ? ba_ld(sb) : F::zero();
-    const bool xa0 = F::is_exact_zero(xa), xb0 = F::is_exact_zero(xb);
-    ya = (sa && (FULL || xa0)) ? ba_load_y<C>(sa, na, xa) : F::zero();
-    yb = (sb && (FULL || xb0)) ? ba_load_y<C>(sb, nb, xb) : F::zero();
-    if (xb0 && F::is_exact_zero(yb))
-        return BA_COPY_A;  // b is the identity
-    if (xa0 && F::is_exact_zero(ya))
-        return BA_COPY_B;  // a is the identity
-    const Fe dx = F::sub(xb, xa);
-    if (F::is_zero(dx)) {
-        if (!FULL) {
-            ya = ba_load_y<C>(sa, na, xa);
-            yb = ba_load_y<C>(sb, nb, xb);
-        }
+    __device__ __forceinline__ uint2 entry(uint64_t q) const
+    {
+        return FIRST ? __ldg(entries + q) : make_uint2((uint32_t)(2 * q), (uint32_t)(2 * q + 1));
+    }
+    __device__ __forceinline__ static bool pad(uint32_t e) { return FIRST && e == PAD_ENTRY; }
+    // (a padding entry reads element 0, and what it read is dropped)
+    __device__ __forceinline__ const uint4 *src(uint32_t e) const
+    {
+        return base + 4 * (size_t)(FIRST ? (pad(e) ? 0u : e & 0x7fffffffu) : e);
+    }
+    __device__ __forceinline__ Fe x(uint32_t e) const { return ldg_fe(src(e), wide); }
+    __device__ __forceinline__ Fe y(uint32_t e) const  // negated for a negative digit; the identity's 0 stays 0
+    {
+        const Fe v = ldg_fe(src(e) + 2, wide);
+        return FIRST && (e >> 31) ? F::neg(v) : v;
+    }
+    // an item that may be the identity (padding, or an x whose low word is 0), or
+    // equal x: the cases that kind() sorts out
+    __device__ __forceinline__ bool rare(const uint2 &e, const Fe &xa, const Fe &xb, const Fe &dx) const
+    {
+        return pad(e.x) || pad(e.y) || xa.w[0] == 0 || xb.w[0] == 0 || F::is_zero(dx);
+    }
+    // kind and denominator of a rare pair (d: x_b - x_a on entry); the coordinates of
+    // a padding item become 0
+    __device__ __forceinline__ int kind(const uint2 &e, Fe &xa, Fe &ya, Fe &xb, Fe &yb, Fe &d) const
+    {
+        if (pad(e.x))
+            xa = ya = F::zero();
+        if (pad(e.y))
+            xb = yb = F::zero();
+        if (F::is_exact_zero(xb) && F::is_exact_zero(yb))
+            return BA_COPY_A;  // b is the identity
+        if (F::is_exact_zero(xa) && F::is_exact_zero(ya))
+            return BA_COPY_B;  // a is the identity
+        if (!F::is_zero(d))
+            return BA_ADD;
         if (!F::is_zero(F::sub(yb, ya)) || F::is_zero(ya))
             return BA_ZERO;  // b = -a (or a point of order 2, which doubles to the identity)
         d = F::dbl(ya);  // b = a: double
         return BA_DBL;
     }
-    d = dx;
-    return BA_ADD;
-}
+};
 
 // first output of this thread's warp tile, plus its lane (outputs base + 32 k),
 // in a launch over outputs [E0, E)
@@ -226,101 +245,132 @@ template <class C, bool FIRST>
 __global__ void __launch_bounds__(BA_BT) k_ba_pairs(const uint32_t *__restrict__ lo, const uint32_t *__restrict__ hi,
                                                    uint32_t r, const uint32_t *__restrict__ sorted,
                                                    const uint4 *__restrict__ pts, const uint4 *__restrict__ lvl,
-                                                   uint4 *__restrict__ pre, uint4 *__restrict__ co,
-                                                   uint4 *__restrict__ tot)
+                                                   uint4 *__restrict__ pre, uint4 *__restrict__ tot)
 {
     using F = typename C::F;
-    __shared__ Fe tree[2 * BA_BT];
-    __shared__ Fe cop[2 * BA_BT];
     const uint32_t E0 = ba_first(lo, r), E = __ldg(hi) >> r;  // outputs of this launch
-    const uint32_t t = threadIdx.x;
     if (E0 + (uint64_t)blockIdx.x * BA_BT * BA_K >= E)
         return;  // the whole block is past the launch's outputs
+    const BaInput<C, FIRST> in(sorted, pts, lvl);
     const uint64_t base = ba_tile_base(E0);
     Fe run = F::one();
     bool any = false;
+    if (base < E) {
+        const int kmax = (int)((E - 1 - base) / 32) < BA_K - 1 ? (int)((E - 1 - base) / 32) : BA_K - 1;
+        uint2 e = in.entry(base), next = kmax > 0 ? in.entry(base + 32) : e;
 #pragma unroll 1
-    for (int k = 0; k < BA_K; k++) {
-        const uint64_t q = base + 32 * (uint64_t)k;
-        if (q >= E)
-            break;
-        Fe xa, ya, xb, yb, d;
-        const int kind = ba_item<C, FIRST, false>(sorted, pts, lvl, (uint32_t)q, xa, ya, xb, yb, d);
-        if (kind == BA_ADD || kind == BA_DBL) {
-            store_fe(pre + 2 * q, run);  // exclusive prefix of this output (1 for the first)
-            run = any ? F::mul(run, d) : d;
-            any = true;
+        for (int k = 0; k <= kmax; k++) {
+            const uint64_t q = base + 32 * (uint64_t)k;
+            const uint2 after = k + 2 <= kmax ? in.entry(q + 64) : next;
+            Fe xa = in.x(e.x), xb = in.x(e.y);
+            Fe d = F::sub(xb, xa);
+            int kind = BA_ADD;
+            if (in.rare(e, xa, xb, d)) {
+                Fe ya = in.y(e.x), yb = in.y(e.y);
+                kind = in.kind(e, xa, ya, xb, yb, d);
+            }
+            if (kind <= BA_DBL) {
+                stg_fe(pre + 2 * q, run);  // exclusive prefix of this output (1 for the first)
+                run = any ? F::mul(run, d) : d;
+                any = true;
+            }
+            e = next;
+            next = after;
         }
     }
-    // product tree over the block's thread totals (leaf t at BA_BT + t)
-    tree[BA_BT + t] = run;
-    __syncthreads();
-    for (uint32_t s2 = BA_BT / 2; s2 >= 1; s2 >>= 1) {
-        if (t < s2)
-            tree[s2 + t] = F::mul(tree[2 * (s2 + t)], tree[2 * (s2 + t) + 1]);
-        __syncthreads();
-    }
-    // co-products top-down: cop[node] = product of all leaves outside node's subtree
-    if (t == 0)
-        cop[1] = F::one();
-    __syncthreads();
-    for (uint32_t s2 = 1; s2 < BA_BT; s2 <<= 1) {
-        if (t < s2) {
-            const uint32_t nd = s2 + t;
-            const Fe c = cop[nd];
-            cop[2 * nd] = F::mul(c, tree[2 * nd + 1]);
-            cop[2 * nd + 1] = F::mul(c, tree[2 * nd]);
-        }
-        __syncthreads();
-    }
-    store_fe(co + 2 * ((size_t)blockIdx.x * BA_BT + t), cop[BA_BT + t]);
-    if (t == 0)
-        store_fe(tot + 2 * (size_t)blockIdx.x, tree[1]);
+    stg_fe(tot + 2 * ((size_t)blockIdx.x * BA_BT + threadIdx.x), run);
 }
 
-// one inversion per block total (a block total is never zero: every factor is)
+// The thread totals' inverses, in place (a total is never zero: every factor is not).
+// A block takes BA_G totals per thread: their running products per thread, a
+// product tree over the threads, one inversion, and the way back.  One inversion per
+// BA_G totals without the tree took 85 us for the 524288 totals of an MSM of 2^20
+// points, against 44 (twice as many, K = 16) and less now.
+constexpr int BA_G = 8;
+constexpr int BA_INV_BT = 128;
+
 template <class C>
-__global__ void k_ba_invert(const uint32_t *__restrict__ lo, const uint32_t *__restrict__ hi, uint32_t r,
-                            const uint4 *__restrict__ tot, uint4 *__restrict__ inv)
+__global__ void __launch_bounds__(BA_INV_BT) k_ba_invert(const uint32_t *__restrict__ lo,
+                                                        const uint32_t *__restrict__ hi, uint32_t r, uint4 *tot)
 {
     using F = typename C::F;
+    __shared__ Fe tree[2 * BA_INV_BT], cop[2 * BA_INV_BT];
     const uint32_t E0 = ba_first(lo, r), E = __ldg(hi) >> r;
-    const uint32_t nblk = (uint32_t)(((uint64_t)(E - E0) + BA_BT * BA_K - 1) / (BA_BT * BA_K));
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nblk)
-        return;
-    store_fe(inv + 2 * (size_t)i, F::inv(load_fe(tot + 2 * (size_t)i)));
+    const uint64_t count = (((uint64_t)(E - E0) + BA_BT * BA_K - 1) / (BA_BT * BA_K)) * BA_BT;
+    const uint32_t t = threadIdx.x;
+    const uint64_t first = blockIdx.x * (uint64_t)(BA_G * BA_INV_BT) + t;  // totals first + j BA_INV_BT
+    if (first - t >= count)
+        return;  // the whole block
+    Fe pre[BA_G];  // products of this thread's totals up to j (1 past the end)
+#pragma unroll
+    for (int j = 0; j < BA_G; j++) {
+        const uint64_t i = first + (uint64_t)j * BA_INV_BT;
+        const Fe v = i < count ? load_fe(tot + 2 * i) : F::one();
+        pre[j] = j ? F::mul(pre[j - 1], v) : v;
+    }
+    // product tree over the threads (leaf t at BA_INV_BT + t), then top down
+    // cop[node] = the inverse of the node's product
+    tree[BA_INV_BT + t] = pre[BA_G - 1];
+    __syncthreads();
+    for (uint32_t s = BA_INV_BT / 2; s >= 1; s >>= 1) {
+        if (t < s)
+            tree[s + t] = F::mul(tree[2 * (s + t)], tree[2 * (s + t) + 1]);
+        __syncthreads();
+    }
+    if (t == 0)
+        cop[1] = F::inv(tree[1]);
+    __syncthreads();
+    for (uint32_t s = 1; s < BA_INV_BT; s <<= 1) {
+        if (t < 2 * s) {  // node 2 s + t, by its sibling
+            const uint32_t nd = 2 * s + t;
+            cop[nd] = F::mul(cop[nd >> 1], tree[nd ^ 1]);
+        }
+        __syncthreads();
+    }
+    Fe inv = cop[BA_INV_BT + t];
+#pragma unroll
+    for (int j = BA_G - 1; j >= 0; j--) {
+        const uint64_t i = first + (uint64_t)j * BA_INV_BT;
+        if (i < count) {
+            const Fe v = load_fe(tot + 2 * i);
+            stg_fe(tot + 2 * i, j ? F::mul(inv, pre[j - 1]) : inv);
+            inv = F::mul(inv, v);
+        }
+    }
 }
 
 template <class C, bool FIRST>
 __global__ void __launch_bounds__(BA_BT) k_ba_finish(const uint32_t *__restrict__ lo, const uint32_t *__restrict__ hi,
                                                     uint32_t r, const uint32_t *__restrict__ sorted,
                                                     const uint4 *__restrict__ pts, const uint4 *__restrict__ lvl,
-                                                    const uint4 *__restrict__ pre, const uint4 *__restrict__ co,
-                                                    const uint4 *__restrict__ inv, uint4 *__restrict__ out)
+                                                    const uint4 *__restrict__ pre, const uint4 *__restrict__ tot,
+                                                    uint4 *__restrict__ out)
 {
     using F = typename C::F;
     const uint32_t E0 = ba_first(lo, r), E = __ldg(hi) >> r;
     const uint64_t base = ba_tile_base(E0);
     if (base >= E)
         return;
+    const BaInput<C, FIRST> in(sorted, pts, lvl);
     // 1 / (this thread's total)
-    Fe inv_run = F::mul(load_fe(inv + 2 * (size_t)blockIdx.x),
-                        load_fe(co + 2 * ((size_t)blockIdx.x * BA_BT + threadIdx.x)));
+    Fe inv_run = ldg_fe(tot + 2 * ((size_t)blockIdx.x * BA_BT + threadIdx.x));
     const int kmax = (int)((E - 1 - base) / 32) < BA_K - 1 ? (int)((E - 1 - base) / 32) : BA_K - 1;
+    uint2 e = in.entry(base + 32 * (uint64_t)kmax), next = kmax > 0 ? in.entry(base + 32 * (uint64_t)(kmax - 1)) : e;
 #pragma unroll 1
     for (int k = kmax; k >= 0; k--) {
         const uint64_t q = base + 32 * (uint64_t)k;
-        Fe xa, ya, xb, yb, d;
-        const int kind = ba_item<C, FIRST, true>(sorted, pts, lvl, (uint32_t)q, xa, ya, xb, yb, d);
+        const uint2 after = k >= 2 ? in.entry(q - 64) : next;
+        Fe xa = in.x(e.x), xb = in.x(e.y), ya = in.y(e.x), yb = in.y(e.y);
+        Fe d = F::sub(xb, xa);
+        int kind = BA_ADD;
+        if (in.rare(e, xa, xb, d))
+            kind = in.kind(e, xa, ya, xb, yb, d);
         Fe x3, y3;
-        if (kind == BA_ADD || kind == BA_DBL) {
-            const Fe inv_d = F::mul(inv_run, load_fe(pre + 2 * q));
+        if (kind <= BA_DBL) {
+            const Fe inv_d = F::mul(inv_run, ldg_fe(pre + 2 * q));
             inv_run = F::mul(inv_run, d);
-            Fe num;
-            if (kind == BA_ADD) {
-                num = F::sub(yb, ya);
-            } else {
+            Fe num = F::sub(yb, ya);
+            if (kind == BA_DBL) {
                 const Fe t = F::sub(F::sqr(xa), F::one());
                 num = F::add(F::dbl(t), t);  // 3 x^2 + a, a = -3
                 xb = xa;
@@ -328,19 +378,15 @@ __global__ void __launch_bounds__(BA_BT) k_ba_finish(const uint32_t *__restrict_
             const Fe lam = F::mul(num, inv_d);
             x3 = F::sub(F::sub(F::sqr(lam), xa), xb);
             y3 = F::sub(F::mul(lam, F::sub(xa, x3)), ya);
-        } else if (kind == BA_COPY_A) {
-            x3 = xa;
-            y3 = ya;
-        } else if (kind == BA_COPY_B) {
-            x3 = xb;
-            y3 = yb;
         } else {
-            x3 = F::zero();
-            y3 = F::zero();
+            x3 = kind == BA_COPY_A ? xa : kind == BA_COPY_B ? xb : F::zero();
+            y3 = kind == BA_COPY_A ? ya : kind == BA_COPY_B ? yb : F::zero();
         }
         uint4 *dst = out + 4 * q;
-        store_fe(dst, x3);
-        store_fe(dst + 2, y3);
+        stg_fe(dst, x3);
+        stg_fe(dst + 2, y3);
+        e = next;
+        next = after;
     }
 }
 
@@ -363,12 +409,12 @@ __global__ void __launch_bounds__(128) k_accumulate_level(const uint4 *__restric
         Xyzz acc = (RESUME && d.w) ? load_xyzz(seg_sum + 8 * (size_t)d.z) : G::inf();
         for (uint32_t i = 0; i < d.y; i++) {
             Fe x, y;
-            load_affine(lvl, d.x + i, x, y);
+            load_affine(lvl, d.x + i, x, y, true);
             if (F::is_exact_zero(x) && F::is_exact_zero(y))
                 continue;
             G::add_affine(acc, x, y);
         }
-        store_xyzz(seg_sum + 8 * (size_t)d.z, acc);
+        stg_xyzz(seg_sum + 8 * (size_t)d.z, acc);
     }
 }
 
@@ -913,21 +959,22 @@ cudaError_t msm_tail(Context &ctx, const BatchPlan &p, const BatchBuffers &b)
                 const uint4 *in_lvl = r == 1 ? nullptr : b.ba_lvl[(r - 2) & 1];
                 uint4 *out_lvl = b.ba_lvl[(r - 1) & 1];
                 const uint32_t blocks = std::max<uint32_t>(1, p.ba_blocks[r - 1]);
+                const uint32_t iblocks = (uint32_t)(((uint64_t)blocks * BA_BT + BA_G * BA_INV_BT - 1) / (BA_G * BA_INV_BT));
                 if (r == 1)
                     k_ba_pairs<C, true><<<blocks, BA_BT, 0, st>>>(lo, hi, r, b.sorted, b.points, in_lvl, b.ba_pre,
-                                                                  b.ba_co, b.ba_tot);
+                                                                  b.ba_tot);
                 else
                     k_ba_pairs<C, false><<<blocks, BA_BT, 0, st>>>(lo, hi, r, b.sorted, b.points, in_lvl, b.ba_pre,
-                                                                   b.ba_co, b.ba_tot);
+                                                                   b.ba_tot);
                 HS_LAUNCH_CHECK(ctx);
-                k_ba_invert<C><<<(blocks + 63) / 64, 64, 0, st>>>(lo, hi, r, b.ba_tot, b.ba_inv);
+                k_ba_invert<C><<<iblocks, BA_INV_BT, 0, st>>>(lo, hi, r, b.ba_tot);
                 HS_LAUNCH_CHECK(ctx);
                 if (r == 1)
                     k_ba_finish<C, true><<<blocks, BA_BT, 0, st>>>(lo, hi, r, b.sorted, b.points, in_lvl, b.ba_pre,
-                                                                   b.ba_co, b.ba_inv, out_lvl);
+                                                                   b.ba_tot, out_lvl);
                 else
                     k_ba_finish<C, false><<<blocks, BA_BT, 0, st>>>(lo, hi, r, b.sorted, b.points, in_lvl,
-                                                                    b.ba_pre, b.ba_co, b.ba_inv, out_lvl);
+                                                                    b.ba_pre, b.ba_tot, out_lvl);
                 HS_LAUNCH_CHECK(ctx);
             }
             const int threads = 128;
@@ -1574,7 +1621,7 @@ __global__ void k_fb_expand(const uint4 *__restrict__ gens, size_t n, int c, int
     if (i >= n)
         return;
     Fe x, y;
-    load_affine(gens, (uint32_t)i, x, y);
+    load_affine(gens, (uint32_t)i, x, y, wide_points(gens));
     Xyzz acc = (F::is_exact_zero(x) && F::is_exact_zero(y)) ? G::inf() : G::from_affine(x, y);
     for (int k = 0; k < W; k++) {
         store_xyzz(tmp + 8 * ((size_t)i * W + k), acc);
@@ -1698,7 +1745,7 @@ __global__ void __launch_bounds__(128) k_scalar_mul(const uint4 *__restrict__ sc
     if (i >= n)
         return;
     Fe x, y;
-    load_affine(pts, (uint32_t)i, x, y);
+    load_affine(pts, (uint32_t)i, x, y, wide_points(pts));
     Xyzz Q = G::inf();
     if (!(F::is_exact_zero(x) && F::is_exact_zero(y))) {
         const uint4 sa = __ldg(scalars + 2 * i), sb = __ldg(scalars + 2 * i + 1);

@@ -492,8 +492,7 @@ size_t batch_bytes(const BatchPlan &p)
         b += align256((size_t)p.ba_items[0] * 64);                                            // odd rounds
         b += p.ba_rounds > 1 ? align256((size_t)p.ba_items[1] * 64) : 0;                      // even rounds
         b += align256((size_t)p.ba_items[0] * 32);                                            // prefixes
-        b += align256((size_t)p.ba_blocks[0] * BA_PLAN_BT * 32);                              // co-products
-        b += 2 * align256((size_t)p.ba_blocks[0] * 32);                                       // totals, inverses
+        b += align256((size_t)p.ba_blocks[0] * BA_PLAN_BT * 32);                              // thread totals
         b += 8 * 256;
     }
     return b + 16 * 256;
@@ -528,9 +527,7 @@ bool carve(DeviceArena &a, const BatchPlan &p, BatchBuffers &b)
         if (p.ba_rounds > 1)
             ba_ok = ba_ok && (b.ba_lvl[1] = (uint4 *)a.take((size_t)p.ba_items[1] * 64));
         ba_ok = ba_ok && (b.ba_pre = (uint4 *)a.take((size_t)p.ba_items[0] * 32));
-        ba_ok = ba_ok && (b.ba_co = (uint4 *)a.take((size_t)p.ba_blocks[0] * BA_PLAN_BT * 32));
-        ba_ok = ba_ok && (b.ba_tot = (uint4 *)a.take((size_t)p.ba_blocks[0] * 32));
-        ba_ok = ba_ok && (b.ba_inv = (uint4 *)a.take((size_t)p.ba_blocks[0] * 32));
+        ba_ok = ba_ok && (b.ba_tot = (uint4 *)a.take((size_t)p.ba_blocks[0] * BA_PLAN_BT * 32));
     }
     return b.desc && b.counts && b.offsets && b.seg_off && b.scan_tmp && b.len_hist && b.len_scan && b.sorted &&
            b.segs && b.seg_sum && b.heavy && b.heavy_n && b.redA && b.redC && b.redS && b.out_jac &&
