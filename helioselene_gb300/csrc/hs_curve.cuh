@@ -177,6 +177,29 @@ struct Group {
         return r;
     }
 
+    // r = p + q for operands that are not the identity; 1 when they are equal and 2
+    // when they are opposite (r is then unset).  The operands are dead after the first
+    // six products, so a caller that can get q again keeps fewer registers than with
+    // add().
+    __device__ __forceinline__ static int add_lean(Xyzz &r, const Xyzz &p, const Xyzz &q)
+    {
+        const Fe U1 = F::mul(p.X, q.ZZ);
+        const Fe P = F::sub(F::mul(q.X, p.ZZ), U1);
+        const Fe S1 = F::mul(p.Y, q.ZZZ);
+        const Fe R = F::sub(F::mul(q.Y, p.ZZZ), S1);
+        const Fe zz = F::mul(p.ZZ, q.ZZ), zzz = F::mul(p.ZZZ, q.ZZZ);
+        if (F::is_zero(P))
+            return F::is_zero(R) ? 1 : 2;
+        const Fe PP = F::sqr(P);
+        const Fe Q = F::mul(U1, PP);
+        const Fe PPP = F::mul(P, PP);
+        r.ZZ = F::mul(zz, PP);
+        r.ZZZ = F::mul(zzz, PPP);
+        r.X = F::sub(F::sub(F::sqr(R), PPP), F::dbl(Q));
+        r.Y = F::sub(F::mul(R, F::sub(Q, r.X)), F::mul(S1, PPP));
+        return 0;
+    }
+
     __device__ __forceinline__ static Xyzz neg(const Xyzz &p)
     {
         Xyzz r = p;
