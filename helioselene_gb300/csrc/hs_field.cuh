@@ -56,6 +56,11 @@ struct FqParams {
 // F_q 4.56 -> 3.80 and 3.68 -> 2.96.  (Karatsuba on 4 x 4 halves saves 16
 // products for about 70 adds: 2.84.  Limbs of 29 bits in 64-bit columns: 3.64.)
 
+// Every output of these statements is early-clobbered (&): a statement is many
+// instructions, and without it an output may share the register of an input of the
+// same value -- a zero accumulator and a zero operand, as in the square of the
+// constant one, which then came out as 39.
+
 // acc[0..2N-1] += sum_k a[2k] b 2^(64k), k < N; with CARRY, acc[2N] = the carry out
 // (without, the caller's bound says there is none)
 template <int N, bool CARRY>
@@ -73,8 +78,8 @@ __device__ __forceinline__ void mad_chain(uint32_t *acc, const uint32_t *a, uint
             "madc.hi.cc.u32 %7, %12, %13, %7;\n\t"
             "addc.u32       %8, 0, 0;\n\t"
             "}"
-            : "+r"(acc[0]), "+r"(acc[1]), "+r"(acc[2]), "+r"(acc[3]), "+r"(acc[4]), "+r"(acc[5]), "+r"(acc[6]),
-              "+r"(acc[7]), "=r"(acc[8])
+            : "+&r"(acc[0]), "+&r"(acc[1]), "+&r"(acc[2]), "+&r"(acc[3]), "+&r"(acc[4]), "+&r"(acc[5]), "+&r"(acc[6]),
+              "+&r"(acc[7]), "=&r"(acc[8])
             : "r"(a[0]), "r"(a[2]), "r"(a[4]), "r"(a[6]), "r"(b));
     else if (N == 4)
         asm("{\n\t"
@@ -87,8 +92,8 @@ __device__ __forceinline__ void mad_chain(uint32_t *acc, const uint32_t *a, uint
             "madc.lo.cc.u32 %6, %11, %12, %6;\n\t"
             "madc.hi.u32    %7, %11, %12, %7;\n\t"
             "}"
-            : "+r"(acc[0]), "+r"(acc[1]), "+r"(acc[2]), "+r"(acc[3]), "+r"(acc[4]), "+r"(acc[5]), "+r"(acc[6]),
-              "+r"(acc[7])
+            : "+&r"(acc[0]), "+&r"(acc[1]), "+&r"(acc[2]), "+&r"(acc[3]), "+&r"(acc[4]), "+&r"(acc[5]), "+&r"(acc[6]),
+              "+&r"(acc[7])
             : "r"(a[0]), "r"(a[2]), "r"(a[4]), "r"(a[6]), "r"(b));
     else if (N == 3 && CARRY)
         asm("{\n\t"
@@ -100,7 +105,7 @@ __device__ __forceinline__ void mad_chain(uint32_t *acc, const uint32_t *a, uint
             "madc.hi.cc.u32 %5, %9, %10, %5;\n\t"
             "addc.u32       %6, 0, 0;\n\t"
             "}"
-            : "+r"(acc[0]), "+r"(acc[1]), "+r"(acc[2]), "+r"(acc[3]), "+r"(acc[4]), "+r"(acc[5]), "=r"(acc[6])
+            : "+&r"(acc[0]), "+&r"(acc[1]), "+&r"(acc[2]), "+&r"(acc[3]), "+&r"(acc[4]), "+&r"(acc[5]), "=&r"(acc[6])
             : "r"(a[0]), "r"(a[2]), "r"(a[4]), "r"(b));
     else if (N == 3)
         asm("{\n\t"
@@ -111,7 +116,7 @@ __device__ __forceinline__ void mad_chain(uint32_t *acc, const uint32_t *a, uint
             "madc.lo.cc.u32 %4, %8, %9, %4;\n\t"
             "madc.hi.u32    %5, %8, %9, %5;\n\t"
             "}"
-            : "+r"(acc[0]), "+r"(acc[1]), "+r"(acc[2]), "+r"(acc[3]), "+r"(acc[4]), "+r"(acc[5])
+            : "+&r"(acc[0]), "+&r"(acc[1]), "+&r"(acc[2]), "+&r"(acc[3]), "+&r"(acc[4]), "+&r"(acc[5])
             : "r"(a[0]), "r"(a[2]), "r"(a[4]), "r"(b));
     else if (N == 2 && CARRY)
         asm("{\n\t"
@@ -121,7 +126,7 @@ __device__ __forceinline__ void mad_chain(uint32_t *acc, const uint32_t *a, uint
             "madc.hi.cc.u32 %3, %6, %7, %3;\n\t"
             "addc.u32       %4, 0, 0;\n\t"
             "}"
-            : "+r"(acc[0]), "+r"(acc[1]), "+r"(acc[2]), "+r"(acc[3]), "=r"(acc[4])
+            : "+&r"(acc[0]), "+&r"(acc[1]), "+&r"(acc[2]), "+&r"(acc[3]), "=&r"(acc[4])
             : "r"(a[0]), "r"(a[2]), "r"(b));
     else if (N == 2)
         asm("{\n\t"
@@ -130,7 +135,7 @@ __device__ __forceinline__ void mad_chain(uint32_t *acc, const uint32_t *a, uint
             "madc.lo.cc.u32 %2, %5, %6, %2;\n\t"
             "madc.hi.u32    %3, %5, %6, %3;\n\t"
             "}"
-            : "+r"(acc[0]), "+r"(acc[1]), "+r"(acc[2]), "+r"(acc[3])
+            : "+&r"(acc[0]), "+&r"(acc[1]), "+&r"(acc[2]), "+&r"(acc[3])
             : "r"(a[0]), "r"(a[2]), "r"(b));
     else if (N == 1 && CARRY)
         asm("{\n\t"
@@ -138,14 +143,14 @@ __device__ __forceinline__ void mad_chain(uint32_t *acc, const uint32_t *a, uint
             "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
             "addc.u32       %2, 0, 0;\n\t"
             "}"
-            : "+r"(acc[0]), "+r"(acc[1]), "=r"(acc[2])
+            : "+&r"(acc[0]), "+&r"(acc[1]), "=&r"(acc[2])
             : "r"(a[0]), "r"(b));
     else
         asm("{\n\t"
             "mad.lo.cc.u32  %0, %2, %3, %0;\n\t"
             "madc.hi.u32    %1, %2, %3, %1;\n\t"
             "}"
-            : "+r"(acc[0]), "+r"(acc[1])
+            : "+&r"(acc[0]), "+&r"(acc[1])
             : "r"(a[0]), "r"(b));
 }
 __device__ __forceinline__ void mul_pair(uint32_t *acc, uint32_t a, uint32_t b)
@@ -215,7 +220,7 @@ __device__ __forceinline__ uint32_t add8(uint32_t *r, const uint32_t *x, const u
     asm("add.cc.u32  %0, %9, %17;\n\taddc.cc.u32 %1, %10, %18;\n\taddc.cc.u32 %2, %11, %19;\n\taddc.cc.u32 %3, %12, %20;\n\t"
         "addc.cc.u32 %4, %13, %21;\n\taddc.cc.u32 %5, %14, %22;\n\taddc.cc.u32 %6, %15, %23;\n\taddc.cc.u32 %7, %16, %24;\n\t"
         "addc.u32 %8, 0, 0;"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(c)
+        : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7]), "=&r"(c)
         : "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(x[4]), "r"(x[5]), "r"(x[6]), "r"(x[7]), "r"(y[0]), "r"(y[1]),
           "r"(y[2]), "r"(y[3]), "r"(y[4]), "r"(y[5]), "r"(y[6]), "r"(y[7]));
     return c;
@@ -229,7 +234,7 @@ __device__ __forceinline__ uint32_t sub8(uint32_t *r, const uint32_t *x, const u
         "subc.cc.u32 %0, %9, %17;\n\tsubc.cc.u32 %1, %10, %18;\n\tsubc.cc.u32 %2, %11, %19;\n\tsubc.cc.u32 %3, %12, %20;\n\t"
         "subc.cc.u32 %4, %13, %21;\n\tsubc.cc.u32 %5, %14, %22;\n\tsubc.cc.u32 %6, %15, %23;\n\tsubc.cc.u32 %7, %16, %24;\n\t"
         "subc.u32 %8, 0, 0;"
-        : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7]), "+r"(m)
+        : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7]), "+&r"(m)
         : "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(x[4]), "r"(x[5]), "r"(x[6]), "r"(x[7]), "r"(y[0]), "r"(y[1]),
           "r"(y[2]), "r"(y[3]), "r"(y[4]), "r"(y[5]), "r"(y[6]), "r"(y[7]));
     return m;
@@ -238,12 +243,25 @@ __device__ __forceinline__ uint32_t sub8(uint32_t *r, const uint32_t *x, const u
 // t[0..14] += o[0..14] (no carry out by the caller's bound)
 __device__ __forceinline__ void merge15(uint32_t *t, const uint32_t *o)
 {
-    uint32_t c = add8(t, t, o);
-    asm("add.cc.u32 %7, %7, 0xffffffff;\n\t"
-        "addc.cc.u32 %0, %0, %8;\n\taddc.cc.u32 %1, %1, %9;\n\taddc.cc.u32 %2, %2, %10;\n\taddc.cc.u32 %3, %3, %11;\n\t"
-        "addc.cc.u32 %4, %4, %12;\n\taddc.cc.u32 %5, %5, %13;\n\taddc.u32 %6, %6, %14;\n\t"
-        : "+r"(t[8]), "+r"(t[9]), "+r"(t[10]), "+r"(t[11]), "+r"(t[12]), "+r"(t[13]), "+r"(t[14]), "+r"(c)
-        : "r"(o[8]), "r"(o[9]), "r"(o[10]), "r"(o[11]), "r"(o[12]), "r"(o[13]), "r"(o[14]));
+    asm("add.cc.u32  %0, %0, %15;\n\t"
+        "addc.cc.u32 %1, %1, %16;\n\t"
+        "addc.cc.u32 %2, %2, %17;\n\t"
+        "addc.cc.u32 %3, %3, %18;\n\t"
+        "addc.cc.u32 %4, %4, %19;\n\t"
+        "addc.cc.u32 %5, %5, %20;\n\t"
+        "addc.cc.u32 %6, %6, %21;\n\t"
+        "addc.cc.u32 %7, %7, %22;\n\t"
+        "addc.cc.u32 %8, %8, %23;\n\t"
+        "addc.cc.u32 %9, %9, %24;\n\t"
+        "addc.cc.u32 %10, %10, %25;\n\t"
+        "addc.cc.u32 %11, %11, %26;\n\t"
+        "addc.cc.u32 %12, %12, %27;\n\t"
+        "addc.cc.u32 %13, %13, %28;\n\t"
+        "addc.u32    %14, %14, %29;"
+        : "+&r"(t[0]), "+&r"(t[1]), "+&r"(t[2]), "+&r"(t[3]), "+&r"(t[4]), "+&r"(t[5]), "+&r"(t[6]), "+&r"(t[7]), "+&r"(t[8]),
+          "+&r"(t[9]), "+&r"(t[10]), "+&r"(t[11]), "+&r"(t[12]), "+&r"(t[13]), "+&r"(t[14])
+        : "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]), "r"(o[8]),
+          "r"(o[9]), "r"(o[10]), "r"(o[11]), "r"(o[12]), "r"(o[13]), "r"(o[14]));
 }
 
 template <class P>
@@ -289,8 +307,8 @@ struct Field {
             "addc.cc.u32 %7, %7, 0;\n\t"
             "addc.u32    %8, 0, 0;\n\t"
             "}"
-            : "+r"(r.w[0]), "+r"(r.w[1]), "+r"(r.w[2]), "+r"(r.w[3]), "+r"(r.w[4]), "+r"(r.w[5]), "+r"(r.w[6]),
-              "+r"(r.w[7]), "=r"(cy)
+            : "+&r"(r.w[0]), "+&r"(r.w[1]), "+&r"(r.w[2]), "+&r"(r.w[3]), "+&r"(r.w[4]), "+&r"(r.w[5]), "+&r"(r.w[6]),
+              "+&r"(r.w[7]), "=&r"(cy)
             : "r"(C0 & mask), "r"(C1 & mask), "r"(C2 & mask), "r"(C3 & mask));
         return cy;
     }
@@ -309,8 +327,8 @@ struct Field {
             "subc.cc.u32 %7, %7, 0;\n\t"
             "subc.u32    %8, 0, 0;\n\t"
             "}"
-            : "+r"(r.w[0]), "+r"(r.w[1]), "+r"(r.w[2]), "+r"(r.w[3]), "+r"(r.w[4]), "+r"(r.w[5]), "+r"(r.w[6]),
-              "+r"(r.w[7]), "=r"(bw)
+            : "+&r"(r.w[0]), "+&r"(r.w[1]), "+&r"(r.w[2]), "+&r"(r.w[3]), "+&r"(r.w[4]), "+&r"(r.w[5]), "+&r"(r.w[6]),
+              "+&r"(r.w[7]), "=&r"(bw)
             : "r"(C0 & mask), "r"(C1 & mask), "r"(C2 & mask), "r"(C3 & mask));
         return bw;  // 0 or 0xffffffff
     }
@@ -354,14 +372,14 @@ struct Field {
         uint32_t more;
         if (P::NC == 1) {
             asm("mad.lo.cc.u32 %0, %3, %4, %0;\n\taddc.cc.u32 %1, %1, 0;\n\taddc.u32 %2, 0, 0;"
-                : "+r"(r.w[0]), "+r"(r.w[1]), "=r"(more)
+                : "+&r"(r.w[0]), "+&r"(r.w[1]), "=&r"(more)
                 : "r"(cy), "r"(C0));
             if (more)
                 carry_from<2>(r);
         } else {
             asm("mad.lo.cc.u32 %0, %6, %7, %0;\n\tmadc.lo.cc.u32 %1, %6, %8, %1;\n\tmadc.lo.cc.u32 %2, %6, %9, %2;\n\t"
                 "madc.lo.cc.u32 %3, %6, %10, %3;\n\taddc.cc.u32 %4, %4, 0;\n\taddc.u32 %5, 0, 0;"
-                : "+r"(r.w[0]), "+r"(r.w[1]), "+r"(r.w[2]), "+r"(r.w[3]), "+r"(r.w[4]), "=r"(more)
+                : "+&r"(r.w[0]), "+&r"(r.w[1]), "+&r"(r.w[2]), "+&r"(r.w[3]), "+&r"(r.w[4]), "=&r"(more)
                 : "r"(cy), "r"(C0), "r"(C1), "r"(C2), "r"(C3));
             if (more)
                 carry_from<5>(r);
@@ -373,14 +391,14 @@ struct Field {
         uint32_t more;
         if (P::NC == 1) {
             asm("sub.cc.u32 %0, %0, %3;\n\tsubc.cc.u32 %1, %1, 0;\n\tsubc.u32 %2, 0, 0;"
-                : "+r"(r.w[0]), "+r"(r.w[1]), "=r"(more)
+                : "+&r"(r.w[0]), "+&r"(r.w[1]), "=&r"(more)
                 : "r"(C0 & mask));
             if (more)
                 borrow_from<2>(r);
         } else {
             asm("sub.cc.u32 %0, %0, %6;\n\tsubc.cc.u32 %1, %1, %7;\n\tsubc.cc.u32 %2, %2, %8;\n\tsubc.cc.u32 %3, %3, %9;\n\t"
                 "subc.cc.u32 %4, %4, 0;\n\tsubc.u32 %5, 0, 0;"
-                : "+r"(r.w[0]), "+r"(r.w[1]), "+r"(r.w[2]), "+r"(r.w[3]), "+r"(r.w[4]), "=r"(more)
+                : "+&r"(r.w[0]), "+&r"(r.w[1]), "+&r"(r.w[2]), "+&r"(r.w[3]), "+&r"(r.w[4]), "=&r"(more)
                 : "r"(C0 & mask), "r"(C1 & mask), "r"(C2 & mask), "r"(C3 & mask));
             if (more)
                 borrow_from<5>(r);
@@ -400,8 +418,8 @@ struct Field {
         asm("sub.cc.u32  %0, %9, %17;\n\tsubc.cc.u32 %1, %10, %18;\n\tsubc.cc.u32 %2, %11, %19;\n\tsubc.cc.u32 %3, %12, %20;\n\t"
             "subc.cc.u32 %4, %13, %21;\n\tsubc.cc.u32 %5, %14, %22;\n\tsubc.cc.u32 %6, %15, %23;\n\tsubc.cc.u32 %7, %16, %24;\n\t"
             "subc.u32 %8, 0, 0;"
-            : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]), "=r"(r.w[4]), "=r"(r.w[5]), "=r"(r.w[6]), "=r"(r.w[7]),
-              "=r"(m)
+            : "=&r"(r.w[0]), "=&r"(r.w[1]), "=&r"(r.w[2]), "=&r"(r.w[3]), "=&r"(r.w[4]), "=&r"(r.w[5]), "=&r"(r.w[6]), "=&r"(r.w[7]),
+              "=&r"(m)
             : "r"(a.w[0]), "r"(a.w[1]), "r"(a.w[2]), "r"(a.w[3]), "r"(a.w[4]), "r"(a.w[5]), "r"(a.w[6]), "r"(a.w[7]),
               "r"(b.w[0]), "r"(b.w[1]), "r"(b.w[2]), "r"(b.w[3]), "r"(b.w[4]), "r"(b.w[5]), "r"(b.w[6]), "r"(b.w[7]));
         sub_c(r, m);
@@ -422,7 +440,7 @@ struct Field {
         r.w[0] = e[0];
         asm("add.cc.u32  %0, %8, %16;\n\taddc.cc.u32 %1, %9, %17;\n\taddc.cc.u32 %2, %10, %18;\n\taddc.cc.u32 %3, %11, %19;\n\t"
             "addc.cc.u32 %4, %12, %20;\n\taddc.cc.u32 %5, %13, %21;\n\taddc.cc.u32 %6, %14, %22;\n\taddc.u32 %7, %15, %23;"
-            : "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]), "=r"(r.w[4]), "=r"(r.w[5]), "=r"(r.w[6]), "=r"(r.w[7]), "=r"(r8)
+            : "=&r"(r.w[1]), "=&r"(r.w[2]), "=&r"(r.w[3]), "=&r"(r.w[4]), "=&r"(r.w[5]), "=&r"(r.w[6]), "=&r"(r.w[7]), "=&r"(r8)
             : "r"(e[1]), "r"(e[2]), "r"(e[3]), "r"(e[4]), "r"(e[5]), "r"(e[6]), "r"(e[7]), "r"(e[8]), "r"(o[0]),
               "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]));
         // r8 c back into the low words; a wrap leaves less than 2^13 in r, so adding c is safe
@@ -430,8 +448,8 @@ struct Field {
         asm("mad.lo.cc.u32 %0, %9, %10, %0;\n\taddc.cc.u32 %1, %1, 0;\n\taddc.cc.u32 %2, %2, 0;\n\t"
             "addc.cc.u32 %3, %3, 0;\n\taddc.cc.u32 %4, %4, 0;\n\taddc.cc.u32 %5, %5, 0;\n\t"
             "addc.cc.u32 %6, %6, 0;\n\taddc.cc.u32 %7, %7, 0;\n\taddc.u32 %8, 0, 0;"
-            : "+r"(r.w[0]), "+r"(r.w[1]), "+r"(r.w[2]), "+r"(r.w[3]), "+r"(r.w[4]), "+r"(r.w[5]), "+r"(r.w[6]),
-              "+r"(r.w[7]), "=r"(cy)
+            : "+&r"(r.w[0]), "+&r"(r.w[1]), "+&r"(r.w[2]), "+&r"(r.w[3]), "+&r"(r.w[4]), "+&r"(r.w[5]), "+&r"(r.w[6]),
+              "+&r"(r.w[7]), "=&r"(cy)
             : "r"(r8), "r"(C0));
         r.w[0] += C0 & (0u - cy);
         return r;
@@ -457,7 +475,7 @@ struct Field {
         mad_chain<2, false>(p + 4, h + 1, C3);
         asm("add.cc.u32 %0, %0, %7;\n\taddc.cc.u32 %1, %1, %8;\n\taddc.cc.u32 %2, %2, %9;\n\taddc.cc.u32 %3, %3, %10;\n\t"
             "addc.cc.u32 %4, %4, %11;\n\taddc.cc.u32 %5, %5, %12;\n\taddc.u32 %6, %6, %13;"
-            : "+r"(p[1]), "+r"(p[2]), "+r"(p[3]), "+r"(p[4]), "+r"(p[5]), "+r"(p[6]), "+r"(p[7])
+            : "+&r"(p[1]), "+&r"(p[2]), "+&r"(p[3]), "+&r"(p[4]), "+&r"(p[5]), "+&r"(p[6]), "+&r"(p[7])
             : "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]));
     }
 
@@ -490,7 +508,7 @@ struct Field {
         uint32_t k;
         asm("mad.lo.cc.u32 %0, %5, %6, %0;\n\tmadc.lo.cc.u32 %1, %5, %7, %1;\n\tmadc.lo.cc.u32 %2, %5, %8, %2;\n\t"
             "madc.lo.cc.u32 %3, %5, %9, %3;\n\taddc.u32 %4, %10, 0;"
-            : "+r"(r.w[4]), "+r"(r.w[5]), "+r"(r.w[6]), "+r"(r.w[7]), "=r"(k)
+            : "+&r"(r.w[4]), "+&r"(r.w[5]), "+&r"(r.w[6]), "+&r"(r.w[7]), "=&r"(k)
             : "r"(c1), "r"(C0), "r"(C1), "r"(C2), "r"(C3), "r"(cy));
         add_c(r, k);
         return r;
@@ -547,8 +565,8 @@ struct Field {
             "madc.lo.cc.u32 %14, %23, %23, %14;\n\t"
             "madc.hi.u32    %15, %23, %23, %15;\n\t"
             "}"
-            : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "+r"(t[6]), "+r"(t[7]),
-              "+r"(t[8]), "+r"(t[9]), "+r"(t[10]), "+r"(t[11]), "+r"(t[12]), "+r"(t[13]), "+r"(t[14]), "+r"(t[15])
+            : "+&r"(t[0]), "+&r"(t[1]), "+&r"(t[2]), "+&r"(t[3]), "+&r"(t[4]), "+&r"(t[5]), "+&r"(t[6]), "+&r"(t[7]),
+              "+&r"(t[8]), "+&r"(t[9]), "+&r"(t[10]), "+&r"(t[11]), "+&r"(t[12]), "+&r"(t[13]), "+&r"(t[14]), "+&r"(t[15])
             : "r"(a.w[0]), "r"(a.w[1]), "r"(a.w[2]), "r"(a.w[3]), "r"(a.w[4]), "r"(a.w[5]), "r"(a.w[6]), "r"(a.w[7]));
         return reduce_wide(t);
     }
@@ -597,8 +615,8 @@ struct Field {
             "subc.cc.u32 %7, %16, %24;\n\t"
             "subc.u32    %8, 0, 0;\n\t"
             "}"
-            : "=r"(d.w[0]), "=r"(d.w[1]), "=r"(d.w[2]), "=r"(d.w[3]), "=r"(d.w[4]), "=r"(d.w[5]), "=r"(d.w[6]),
-              "=r"(d.w[7]), "=r"(bw)
+            : "=&r"(d.w[0]), "=&r"(d.w[1]), "=&r"(d.w[2]), "=&r"(d.w[3]), "=&r"(d.w[4]), "=&r"(d.w[5]), "=&r"(d.w[6]),
+              "=&r"(d.w[7]), "=&r"(bw)
             : "r"(v.w[0]), "r"(v.w[1]), "r"(v.w[2]), "r"(v.w[3]), "r"(v.w[4]), "r"(v.w[5]), "r"(v.w[6]),
               "r"(v.w[7]), "r"(M0), "r"(M1), "r"(M2), "r"(M3), "r"(M4), "r"(M5), "r"(M6), "r"(M7));
         return bw ? v : d;
