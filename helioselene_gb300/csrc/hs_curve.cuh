@@ -208,6 +208,57 @@ struct Group {
         return r;
     }
 
+    // ---- Jacobian points (x = X/Z^2, y = Y/Z^3; the identity is Z exactly zero), for
+    // chains of doublings: dbl-2001-b is 3M + 5S against XYZZ's 7M + 2S ----
+    struct Jac {
+        Fe X, Y, Z;
+    };
+    // an addend with the powers of its Z that an addition needs
+    struct JacEntry {
+        Fe X, Y, Z, ZZ, ZZZ;
+    };
+    __device__ __forceinline__ static bool is_inf(const Jac &p) { return F::is_exact_zero(p.Z); }
+    __device__ __forceinline__ static Jac jac_inf() { return Jac{F::one(), F::one(), F::zero()}; }
+
+    // 2p, a = -3 (the identity's Z stays exactly zero)
+    __device__ __forceinline__ static Jac dbl(const Jac &p)
+    {
+        const Fe delta = F::sqr(p.Z), gamma = F::sqr(p.Y);
+        const Fe t = F::mul(F::sub(p.X, delta), F::add(p.X, delta));
+        const Fe alpha = F::add(F::dbl(t), t);
+        Jac r;
+        r.Z = F::sub(F::sub(F::sqr(F::add(p.Y, p.Z)), gamma), delta);
+        const Fe g2 = F::dbl(gamma);
+        const Fe b4 = F::dbl(F::mul(p.X, g2));  // 4 X gamma
+        r.X = F::sub(F::sqr(alpha), F::dbl(b4));
+        r.Y = F::sub(F::mul(alpha, F::sub(b4, r.X)), F::dbl(F::sqr(g2)));
+        if (F::is_zero(r.Z))  // y = 0: no such point on a prime-order curve, kept complete
+            r.Z = F::zero();
+        return r;
+    }
+
+    // p + (q, or -q), complete
+    __device__ __forceinline__ static Jac add(const Jac &p, const JacEntry &q, bool negate)
+    {
+        const Fe y2 = negate ? F::neg(q.Y) : q.Y;
+        if (F::is_exact_zero(q.ZZ))
+            return p;
+        if (is_inf(p))
+            return Jac{q.X, y2, q.Z};
+        const Fe z1z1 = F::sqr(p.Z);
+        const Fe U1 = F::mul(p.X, q.ZZ), S1 = F::mul(p.Y, q.ZZZ);
+        const Fe H = F::sub(F::mul(q.X, z1z1), U1);
+        const Fe R = F::sub(F::mul(y2, F::mul(p.Z, z1z1)), S1);
+        if (F::is_zero(H))
+            return F::is_zero(R) ? dbl(p) : jac_inf();
+        const Fe HH = F::sqr(H), HHH = F::mul(H, HH), V = F::mul(U1, HH);
+        Jac r;
+        r.Z = F::mul(F::mul(p.Z, q.Z), H);
+        r.X = F::sub(F::sub(F::sqr(R), HHH), F::dbl(V));
+        r.Y = F::mul_sub(R, F::sub(V, r.X), S1, HHH);
+        return r;
+    }
+
     // XYZZ -> Jacobian without inversion: Z = ZZ*ZZZ, X = X*ZZ*ZZZ^2, Y = Y*ZZ^3*ZZZ^2.
     // Identity -> (1:1:0), the reference's encoding (helios/include/helios_ops.h:45-50).
     __device__ static void to_jacobian(Fe &X, Fe &Y, Fe &Z, const Xyzz &p)

@@ -1785,12 +1785,15 @@ cudaError_t join(Context &ctx, const uint32_t *d_a, const uint32_t *d_b, size_t 
 // independent variable-time scalar multiplications s_i * P_i
 // (helios/include/helios_scalarmult_vartime.h:39-57, the n = 1 case of the MSM)
 // ---------------------------------------------------------------------------
-// One thread per pair: signed 4-bit digits d_0..d_64 in [-8, 8] (the recode of
-// the MSM with c = 4, carry kept), a table of P..8P in XYZZ, then from the top
-// digit four doublings and one addition of +-|d| P per digit.
+// One thread per pair, from the top digit four doublings and one addition per signed
+// 4-bit digit.  With s' = s + 8 (1 + 16 + 16^2 + ...) the digits are the nibbles of s'
+// less 8, in [-8, 7], and the carry of s' is the top digit.  The chain is in
+// Jacobian coordinates (a doubling 3M + 5S against XYZZ's 7M + 2S, and 24 registers
+// less); the table P..8P keeps each entry's Z^2 and Z^3, so that an addition is
+// 11M + 3S.  2^17 pairs on F_p: 4.50 ms in XYZZ, 4.02 so (4.15 with three blocks per SM).
 template <class C>
-__global__ void __launch_bounds__(128) k_scalar_mul(const uint4 *__restrict__ scalars, const uint4 *__restrict__ pts,
-                                                   size_t n, uint32_t *__restrict__ out)
+__global__ void __launch_bounds__(128, 4) k_scalar_mul(const uint4 *__restrict__ scalars, const uint4 *__restrict__ pts,
+                                                      size_t n, uint32_t *__restrict__ out)
 {
     using G = Group<C>;
     using F = typename C::F;
@@ -1799,40 +1802,42 @@ __global__ void __launch_bounds__(128) k_scalar_mul(const uint4 *__restrict__ sc
         return;
     Fe x, y;
     load_affine(pts, (uint32_t)i, x, y, wide_points(pts));
-    Xyzz Q = G::inf();
+    typename G::Jac Q = G::jac_inf();
     if (!(F::is_exact_zero(x) && F::is_exact_zero(y))) {
         const uint4 sa = __ldg(scalars + 2 * i), sb = __ldg(scalars + 2 * i + 1);
         const uint32_t s[8] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y, sb.z, sb.w};
-        int8_t d[65];
-        uint32_t carry = 0;
-#pragma unroll
-        for (int k = 0; k < 65; k++) {
-            const uint32_t v = (k < 64 ? (s[k >> 3] >> (4 * (k & 7))) & 15u : 0u) + carry;
-            if (k < 64 && v >= 8u) {
-                d[k] = (int8_t)((int)v - 16);
-                carry = 1;
-            } else {
-                d[k] = (int8_t)v;
-                carry = 0;
-            }
+        const uint32_t eights[8] = {0x88888888u, 0x88888888u, 0x88888888u, 0x88888888u,
+                                    0x88888888u, 0x88888888u, 0x88888888u, 0x88888888u};
+        uint32_t d[8];
+        const uint32_t top = add8(d, s, eights);
+        typename G::JacEntry T[8];
+        T[0] = typename G::JacEntry{x, y, F::one(), F::one(), F::one()};
+        typename G::Jac P = G::dbl(typename G::Jac{x, y, F::one()});
+        for (int j = 1; j < 8; j++) {
+            if (j > 1)
+                P = G::add(P, T[0], false);
+            const Fe zz = F::sqr(P.Z);
+            T[j] = typename G::JacEntry{P.X, P.Y, P.Z, zz, F::mul(zz, P.Z)};
         }
-        Xyzz T[8];
-        T[0] = G::from_affine(x, y);
-        T[1] = G::dbl(T[0]);
-        for (int j = 2; j < 8; j++) {
-            T[j] = T[j - 1];
-            G::add_affine(T[j], x, y);
-        }
-        for (int k = 64; k >= 0; k--) {
-            if (k < 64)
-                for (int b = 0; b < 4; b++)
-                    Q = G::dbl(Q);
-            const int dk = d[k];
+        if (top)
+            Q = typename G::Jac{x, y, F::one()};
+#pragma unroll 1
+        for (int k = 63; k >= 0; k--) {
+#pragma unroll 1
+            for (int b = 0; b < 4; b++)
+                Q = G::dbl(Q);
+            const int dk = (int)((d[k >> 3] >> (4 * (k & 7))) & 15u) - 8;
             if (dk != 0)
-                Q = G::add(Q, dk > 0 ? T[dk - 1] : G::neg(T[-dk - 1]));
+                Q = G::add(Q, T[(dk > 0 ? dk : -dk) - 1], dk < 0);
         }
     }
-    store_jacobian_canon<C>(out + 24 * i, Q);
+    const bool inf = G::is_inf(Q);
+    const Fe v[3] = {F::canon(inf ? F::one() : Q.X), F::canon(inf ? F::one() : Q.Y), F::canon(Q.Z)};
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+#pragma unroll
+        for (int w = 0; w < 8; w++)
+            out[24 * i + 8 * c + w] = v[c].w[w];
 }
 
 template <class C>
