@@ -152,6 +152,11 @@ constexpr uint32_t SORT_SMEM_MAX_B = 32768;
 constexpr int SORT_THREADS = 1024;
 constexpr uint32_t SORT_MIN_POINTS_PER_BLOCK = 8192;  // below this average per block: the global-atomic sort
 
+// the single-block sort of a small plan: buckets and entries it takes
+constexpr uint32_t SMALL_SORT_MAX_NB = 8192;
+constexpr uint64_t SMALL_SORT_MAX_ENTRIES = 98304;
+constexpr size_t SMALL_SORT_SMEM = (2 * (size_t)SMALL_SORT_MAX_NB + 160) * 4;
+
 // A run of MSMs sharing one window width (one templated recode launch).
 struct WindowClass {
     int c;
@@ -177,6 +182,15 @@ struct BatchPlan {
     uint64_t cnt_len = 0;       // per-block bucket counts (shared-memory path)
     bool global_sort = false;   // keep the global-atomic sort (no digit and count buffers)
     bool smem_sort() const { return !global_sort && max_B <= SORT_SMEM_MAX_B; }
+    // One MSM whose buckets and entries a single block sorts in shared memory
+    // (k_sort_small): one launch for the recode, the sort and the segments instead of
+    // eleven.  A call of 16 points from host records: 316 us with the general sort, 291 so;
+    // the pair of calls of 602 and 345 points: 796 and 750.
+    bool small_sort() const
+    {
+        return M == 1 && NB <= SMALL_SORT_MAX_NB && entries_bound <= SMALL_SORT_MAX_ENTRIES && !ba_rounds &&
+               !part_slice;
+    }
     uint32_t L = 0;             // max entries per accumulation segment
     uint32_t max_entries = 0;
     uint32_t max_segs = 0;

@@ -1044,6 +1044,11 @@ cudaError_t msm_tail(Context &ctx, const BatchPlan &p, const BatchBuffers &b)
         const uint64_t want = (p.max_segs + 31) / 32;
         const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)ctx.sm_count * 8));
         const size_t nh = (size_t)(p.L + 1) * p.hist_blocks;
+        if (b.ready[0]) {  // host inputs: the bases arrive on another stream
+            const cudaError_t e = cudaStreamWaitEvent(st, b.ready[0], ctx.capturing_host ? cudaEventWaitExternal : 0);
+            if (e != cudaSuccess)
+                return e;
+        }
         cudaEvent_t ev0 = nullptr;
         prof_begin(ctx, &ev0);
         k_accumulate_quads<C><<<blocks, 128, 0, st>>>(b.segs, b.len_scan, b.len_scan + nh, b.sorted, b.points,
@@ -1077,23 +1082,34 @@ cudaError_t msm_tail(Context &ctx, const BatchPlan &p, const BatchBuffers &b)
             prof_end(ctx, ev0, j == 0 ? p.entries_pinned : 0);
         }
     }
-    // 3. merge multi-segment buckets
-    {
-        cudaError_t e = cudaMemsetAsync(b.heavy_n, 0, sizeof(uint32_t), st);
-        if (e != cudaSuccess)
-            return e;
+    // 3. merge multi-segment buckets: a bucket holds at most one entry per point (per
+    //    point and window in a fixed-base MSM), so plans of few points have none, or
+    //    none of more than HEAVY_MIN segments
+    constexpr uint32_t HEAVY_MIN = 8;
+    uint64_t most = 0;
+    for (const MsmDesc &d : p.msms)
+        most = std::max<uint64_t>(most, (uint64_t)d.n * (d.fixed ? d.w_cnt : 1u));
+    if (p.ba_rounds || most > p.L) {
+        const bool any_heavy = p.ba_rounds || most > (uint64_t)HEAVY_MIN * p.L;
+        if (any_heavy) {
+            cudaError_t e = cudaMemsetAsync(b.heavy_n, 0, sizeof(uint32_t), st);
+            if (e != cudaSuccess)
+                return e;
+        }
         const int threads = 256;
         if (small) {
             const unsigned mb = (unsigned)std::max<uint32_t>(1, std::min<uint32_t>((p.NB + 31) / 32,
                                                                                    (uint32_t)ctx.sm_count * 8));
-            k_merge_quads<C><<<mb, 128, 0, st>>>(b.seg_off, p.NB, b.seg_sum, b.heavy, b.heavy_n, 8);
+            k_merge_quads<C><<<mb, 128, 0, st>>>(b.seg_off, p.NB, b.seg_sum, b.heavy, b.heavy_n, HEAVY_MIN);
         } else {
             k_merge_light<C><<<(p.NB + threads - 1) / threads, threads, 0, st>>>(b.seg_off, p.NB, b.seg_sum,
-                                                                               b.heavy, b.heavy_n, 8);
+                                                                               b.heavy, b.heavy_n, HEAVY_MIN);
         }
         HS_LAUNCH_CHECK(ctx);
-        k_merge_heavy<C><<<ctx.sm_count, HEAVY_THREADS, 0, st>>>(b.seg_off, b.heavy, b.heavy_n, b.seg_sum);
-        HS_LAUNCH_CHECK(ctx);
+        if (any_heavy) {
+            k_merge_heavy<C><<<ctx.sm_count, HEAVY_THREADS, 0, st>>>(b.seg_off, b.heavy, b.heavy_n, b.seg_sum);
+            HS_LAUNCH_CHECK(ctx);
+        }
     }
     // 4. bucket reduction: group running sums, then one block per window; a
     //    plan of few windows of at most WQ_MAX_B buckets reduces each window on

@@ -1125,6 +1125,100 @@ __global__ void __launch_bounds__(SEG_HIST_THREADS) k_seg_scatter(const uint32_t
         emit_segments(cur + (L + 1), L, pl.start1, pl.c1, dest, dest + 1, 0u, segs);
 }
 
+// signed digits of one scalar for a window width known at run time (the rule of
+// recode_one): fn(window, magnitude, negative) for every emitted nonzero digit
+template <class Fn>
+__device__ __forceinline__ void for_digits(uint32_t s[8], uint32_t c, uint32_t W, uint32_t w_lo, uint32_t w_cnt, Fn fn)
+{
+    const uint32_t B = 1u << (c - 1), mask = (1u << c) - 1u;
+    uint32_t carry = 0;
+    for (uint32_t k = 0; k < W; k++) {
+        const uint32_t v = (s[0] & mask) + carry;
+#pragma unroll
+        for (int i = 0; i < 7; i++)
+            s[i] = __funnelshift_r(s[i], s[i + 1], c);
+        s[7] >>= c;
+        const bool high = k + 1 < W && v >= B;
+        const uint32_t mag = high ? (1u << c) - v : v;
+        carry = high ? 1u : 0u;
+        if (mag != 0 && k - w_lo < w_cnt)
+            fn(k, mag, high);
+    }
+}
+
+// Recode, counting sort and segments of a small plan (BatchPlan::small_sort) on one
+// block: bucket counts and cursors in shared memory, two passes over the scalars.
+__global__ void __launch_bounds__(SCAN_THREADS) k_sort_small(const uint4 *__restrict__ scalars,
+                                                            const MsmDesc *__restrict__ desc, uint32_t NB, uint32_t L,
+                                                            uint32_t *__restrict__ sorted,
+                                                            uint32_t *__restrict__ seg_off, uint4 *__restrict__ segs,
+                                                            uint32_t *__restrict__ seg_lo,
+                                                            uint32_t *__restrict__ seg_hi,
+                                                            const uint32_t *__restrict__ pt_idx)
+{
+    extern __shared__ uint32_t sm[];
+    uint32_t *cnt = sm, *cur = sm + NB, *len = sm + 2 * NB;  // len[0..L]: segments of each length, then their slots
+    __shared__ uint2 tot;
+    const uint32_t t = threadIdx.x;
+    const MsmDesc d = desc[0];
+    for (uint32_t i = t; i < NB; i += SCAN_THREADS)
+        cnt[i] = 0;
+    for (uint32_t i = t; i <= L; i += SCAN_THREADS)
+        len[i] = 0;
+    __syncthreads();
+    const uint32_t wstep = d.fixed ? 0u : d.B;
+    for (uint32_t i = t; i < d.n; i += SCAN_THREADS) {
+        uint32_t s[8];
+        load_scalar(scalars, d.pt_off + i, s);
+        for_digits(s, d.c, d.W, d.w_lo, d.w_cnt,
+                   [&](uint32_t k, uint32_t mag, bool) { atomicAdd(cnt + (k - d.w_lo) * wstep + mag - 1u, 1u); });
+    }
+    __syncthreads();
+    const uint32_t per = (NB + SCAN_THREADS - 1) / SCAN_THREADS, lo = t * per;
+    uint2 v = make_uint2(0, 0);
+    for (uint32_t i = lo; i < lo + per && i < NB; i++) {
+        const uint32_t c = cnt[i], full = c / L, rem = c % L;
+        v.x += c;
+        v.y += full + (rem ? 1u : 0u);
+        if (full)
+            atomicAdd(len + L, full);
+        if (rem)
+            atomicAdd(len + rem, 1u);
+    }
+    uint2 pre = block_excl_scan(v, &tot);
+    __syncthreads();
+    if (t == 0) {
+        uint32_t at = 0;  // longest first
+        for (uint32_t l = L; l > 0; l--) {
+            const uint32_t c = len[l];
+            len[l] = at;
+            at += c;
+        }
+        seg_off[NB] = tot.y;
+        *seg_lo = 0;
+        *seg_hi = tot.y;
+    }
+    __syncthreads();
+    for (uint32_t i = lo; i < lo + per && i < NB; i++) {
+        const uint32_t c = cnt[i];
+        cur[i] = pre.x;
+        seg_off[i] = pre.y;
+        emit_segments(len, L, pre.x, c, pre.y, pre.y + 1, 0u, segs);
+        pre.x += c;
+        pre.y += (c + L - 1) / L;
+    }
+    __syncthreads();
+    for (uint32_t i = t; i < d.n; i += SCAN_THREADS) {
+        uint32_t s[8];
+        load_scalar(scalars, d.pt_off + i, s);
+        const uint32_t pbase = d.fixed ? table_gen(d, pt_idx, d.pt_off + i) * d.W : d.pt_off + i;
+        for_digits(s, d.c, d.W, d.w_lo, d.w_cnt, [&](uint32_t k, uint32_t mag, bool neg) {
+            const uint32_t pos = atomicAdd(cur + (k - d.w_lo) * wstep + mag - 1u, 1u);
+            sorted[pos] = (pbase + (d.fixed ? k : 0u)) | (neg ? 0x80000000u : 0u);
+        });
+    }
+}
+
 static cudaError_t launch_scan(Context &ctx, const uint32_t *in, uint32_t n, uint32_t L, uint32_t *out,
                                uint32_t *out2, uint32_t *tmp, const uint32_t *counts0 = nullptr, uint32_t pad = 0,
                                uint32_t split_nb = 0, uint32_t shift = 0)
@@ -1159,8 +1253,10 @@ cudaError_t sort_smem_attrs(int device)
                                              (int)(SORT_SMEM_MAX_B * 4));
         cudaError_t b = cudaFuncSetAttribute(k_sort_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)(SORT_SMEM_MAX_B * 4));
+        cudaError_t c = cudaFuncSetAttribute(k_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)SMALL_SORT_SMEM);
         cudaSetDevice(prev);
-        err[device] = a != cudaSuccess ? a : b;
+        err[device] = a != cudaSuccess ? a : (b != cudaSuccess ? b : c);
     });
     return err[device];
 }
@@ -1169,9 +1265,18 @@ cudaError_t launch_sort(Context &ctx, const BatchPlan &p, const BatchBuffers &b)
 {
     cudaStream_t st = ctx.stream;
     cudaError_t e;
+    const uint4 *sc = reinterpret_cast<const uint4 *>(b.scalars);
+    if (p.small_sort()) {
+        if ((e = sort_smem_attrs(ctx.device)) != cudaSuccess)
+            return e;
+        const size_t smem = (2 * (size_t)p.NB + p.L + 2) * 4;
+        k_sort_small<<<1, SCAN_THREADS, smem, st>>>(sc, b.desc, p.NB, p.L, b.sorted, b.seg_off, b.segs, b.len_scan,
+                                                    b.len_scan + hist_len(p), b.pt_idx);
+        HS_LAUNCH_CHECK(ctx);
+        return cudaSuccess;
+    }
     if ((e = cudaMemsetAsync(b.counts, 0, (size_t)(p.NB + 1) * 4, st)) != cudaSuccess)
         return e;
-    const uint4 *sc = reinterpret_cast<const uint4 *>(b.scalars);
     // batch-affine plans: every bucket's list padded to a multiple of 2^R with
     // PAD_ENTRY (the identity), and the fold's segments counted on lists 2^R
     // times shorter
