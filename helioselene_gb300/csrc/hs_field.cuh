@@ -647,33 +647,30 @@ struct Field {
 
     __device__ __forceinline__ static bool eq(const Fe &a, const Fe &b) { return is_zero(sub(a, b)); }
 
-    // a^e for e given as eight 32-bit words (4-bit fixed window)
-    __device__ static Fe pow(const Fe &a, const uint32_t e[8])
+    // a^(2^n), n >= 0
+    __device__ __forceinline__ static Fe sqr_n(Fe a, int n)
     {
-        Fe tab[16];
-        tab[0] = one();
-        tab[1] = a;
 #pragma unroll 1
-        for (int i = 2; i < 16; i++)
-            tab[i] = mul(tab[i - 1], a);
-        Fe acc = one();
+        for (int i = 0; i < n; i++)
+            a = sqr(a);
+        return a;
+    }
+
+    // a^(2^k - 1), k >= 1: a run of n ones doubles to 2n by n squarings and one product
+    __device__ static Fe pow_ones(const Fe &a, int k)
+    {
+        Fe r = a;
+        int n = 1;
 #pragma unroll 1
-        for (int i = 63; i >= 0; i--) {
-            acc = sqr(acc);
-            acc = sqr(acc);
-            acc = sqr(acc);
-            acc = sqr(acc);
-            uint32_t nib = (e[i >> 3] >> (4 * (i & 7))) & 15u;
-            if (nib) {
-                Fe m = tab[0];
-#pragma unroll
-                for (int k = 1; k < 16; k++)
-                    if (k == (int)nib)
-                        m = tab[k];
-                acc = mul(acc, m);
+        for (int b = 30 - __clz(k); b >= 0; b--) {
+            r = mul(sqr_n(r, n), r);
+            n *= 2;
+            if ((k >> b) & 1) {
+                r = mul(sqr(r), a);
+                n++;
             }
         }
-        return acc;
+        return r;
     }
 
     // ---- inversion by batched divsteps ----------------------------------------
