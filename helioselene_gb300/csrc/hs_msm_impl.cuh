@@ -8,7 +8,7 @@
 //      contiguously per bucket;
 //   2. k_accumulate: buckets are cut into segments of at most L entries, one
 //      thread sums one segment of affine bases into an XYZZ point;
-//   3. k_merge_light / k_merge_heavy: buckets with several segments are folded
+//   3. k_merge / k_merge_heavy: buckets with several segments are folded
 //      (sequentially when few, by a block-wide tree when many);
 //   4. k_reduce_groups / k_window_chunks / k_window_sum: per window
 //      S = sum_j (j+1) B_j by running sums over groups of 8 buckets, then
@@ -421,60 +421,88 @@ __global__ void __launch_bounds__(128) k_accumulate_level(const uint4 *__restric
 // ---------------------------------------------------------------------------
 // 3. folding buckets that were cut into several segments
 // ---------------------------------------------------------------------------
+// Both kernels work on quads: a bucket's few additions in sequence and a heavy
+// bucket's tree are latency, which one thread's 14 products per addition set: 66 + 70 us
+// for one F_q MSM of 65521 points, 38 + 23 so.
 template <class C>
-__global__ void k_merge_light(const uint32_t *__restrict__ seg_off, uint32_t NB, uint4 *__restrict__ seg_sum,
-                              uint32_t *__restrict__ heavy, uint32_t *__restrict__ heavy_n, uint32_t heavy_min)
+__global__ void __launch_bounds__(128) k_merge(const uint32_t *__restrict__ seg_off, uint32_t NB,
+                                              uint4 *__restrict__ seg_sum, uint32_t *__restrict__ heavy,
+                                              uint32_t *__restrict__ heavy_n, uint32_t heavy_min)
 {
-    using G = Group<C>;
-    const uint32_t kb = blockIdx.x * blockDim.x + threadIdx.x;
-    if (kb >= NB)
-        return;
-    const uint32_t s0 = seg_off[kb], ns = seg_off[kb + 1] - s0;
-    if (ns < 2)
-        return;
-    if (ns > heavy_min) {
-        heavy[atomicAdd(heavy_n, 1u)] = kb;
-        return;
+    using F = typename C::F;
+    using Q = Quad<C>;
+    const Q op(threadIdx.x);
+    const uint32_t stride = gridDim.x * (blockDim.x >> 2);
+    for (uint32_t w = blockIdx.x * (blockDim.x >> 2) + (threadIdx.x >> 5) * 8; w < NB; w += stride) {
+        const uint32_t kb = w + ((threadIdx.x >> 2) & 7);
+        uint32_t s0 = 0, ns = 0;
+        if (kb < NB) {
+            s0 = seg_off[kb];
+            ns = seg_off[kb + 1] - s0;
+            if (ns > heavy_min) {
+                if (op.j == 0)
+                    heavy[atomicAdd(heavy_n, 1u)] = kb;
+                ns = 0;
+            }
+        }
+        const uint32_t most = __reduce_max_sync(Q::ALL, ns);
+        if (most < 2)
+            continue;
+        Fe acc = ns > 1 ? Q::load(seg_sum, s0, op.j) : F::zero();
+        for (uint32_t i = 1; i < most; i++) {
+            const bool take = i < ns;
+            const Fe o = take ? Q::load(seg_sum, s0 + i, op.j) : F::zero();
+            acc = op.template add<false>(acc, o, take);
+        }
+        if (ns > 1)
+            Q::store(seg_sum, s0, op.j, acc);
     }
-    Xyzz acc = load_xyzz(seg_sum + 8 * (size_t)s0);
-    for (uint32_t j = 1; j < ns; j++)
-        acc = G::add(acc, load_xyzz(seg_sum + 8 * (size_t)(s0 + j)));
-    store_xyzz(seg_sum + 8 * (size_t)s0, acc);
 }
 
-constexpr int HEAVY_THREADS = 128;
+constexpr int HEAVY_QUADS = 64;
 
 template <class C>
-__global__ void __launch_bounds__(HEAVY_THREADS) k_merge_heavy(const uint32_t *__restrict__ seg_off,
-                                                              const uint32_t *__restrict__ heavy,
-                                                              const uint32_t *__restrict__ heavy_n,
-                                                              uint4 *__restrict__ seg_sum)
+__global__ void __launch_bounds__(HEAVY_QUADS * 4) k_merge_heavy(const uint32_t *__restrict__ seg_off,
+                                                                const uint32_t *__restrict__ heavy,
+                                                                const uint32_t *__restrict__ heavy_n,
+                                                                uint4 *__restrict__ seg_sum)
 {
-    using G = Group<C>;
-    __shared__ uint4 sh[HEAVY_THREADS * 8];
+    using F = typename C::F;
+    using Q = Quad<C>;
+    __shared__ uint4 sh[HEAVY_QUADS * 8];
+    const Q op(threadIdx.x);
+    const uint32_t g = threadIdx.x >> 2;
     const uint32_t cnt = *heavy_n;
     for (uint32_t h = blockIdx.x; h < cnt; h += gridDim.x) {
         const uint32_t kb = heavy[h];
         const uint32_t s0 = seg_off[kb], ns = seg_off[kb + 1] - s0;
-        Xyzz acc = G::inf();
-        for (uint32_t j = threadIdx.x; j < ns; j += HEAVY_THREADS)
-            acc = G::add(acc, load_xyzz(seg_sum + 8 * (size_t)(s0 + j)));
-        store_xyzz(sh + 8 * threadIdx.x, acc);
+        Fe acc = g < ns ? Q::load(seg_sum, s0 + g, op.j) : F::zero();
+        const uint32_t first = g & ~7u;  // the warp's first quad: its quads loop together
+        for (uint32_t i = first + HEAVY_QUADS; i < ns; i += HEAVY_QUADS) {
+            const uint32_t mine = i + (g - first);
+            const bool take = mine < ns;
+            const Fe o = take ? Q::load(seg_sum, s0 + mine, op.j) : F::zero();
+            acc = op.template add<false>(acc, o, take);
+        }
+        Q::store(sh, g, op.j, acc);
         __syncthreads();
-        // the tree spans only the threads that hold a segment (a power of two)
+        // the tree spans only the quads that hold a segment (a power of two)
         uint32_t width = 1;
-        while (width < ns && width < HEAVY_THREADS)
+        while (width < ns && width < (uint32_t)HEAVY_QUADS)
             width <<= 1;
         for (uint32_t stride = width / 2; stride > 0; stride >>= 1) {
-            if (threadIdx.x < stride) {
-                Xyzz a = load_xyzz(sh + 8 * threadIdx.x);
-                Xyzz b = load_xyzz(sh + 8 * (threadIdx.x + stride));
-                store_xyzz(sh + 8 * threadIdx.x, G::add(a, b));
+            if (first < stride) {  // whole warps
+                const bool take = g < stride;
+                const Fe o = take ? Q::load(sh, g + stride, op.j) : F::zero();
+                acc = op.template add<false>(acc, o, take);
             }
             __syncthreads();
+            if (g < stride)
+                Q::store(sh, g, op.j, acc);
+            __syncthreads();
         }
-        if (threadIdx.x == 0)
-            store_xyzz(seg_sum + 8 * (size_t)s0, load_xyzz(sh));
+        if (g == 0)
+            Q::store(seg_sum, s0, op.j, acc);
         __syncthreads();
     }
 }
@@ -891,11 +919,9 @@ __global__ void __launch_bounds__(WQ_QUADS * 4) k_window_quads(const uint32_t *_
         Q::store(S, s, op.j, v);
 }
 
-// Bucket accumulation and merges of small plans on quads (a mixed addition is
-// 4 product stages against 10 products on one thread): one quad per segment,
-// then one quad per bucket of 2..8 segments (more go to the heavy-bucket list as
-// in k_merge_light).  16 product slots per entry against 10, so only for plans
-// of at most ACC_QUADS_MAX_ENTRIES entries.
+// Bucket accumulation of small plans on quads (a mixed addition is 4 product stages
+// against 10 products on one thread), one quad per segment.  16 product slots per
+// entry against 10, so only for plans of at most ACC_QUADS_MAX_ENTRIES entries.
 constexpr uint64_t ACC_QUADS_MAX_ENTRIES = 98304;
 
 template <class C>
@@ -943,45 +969,10 @@ __global__ void __launch_bounds__(128) k_accumulate_quads(const uint4 *__restric
 }
 
 template <class C>
-__global__ void __launch_bounds__(128) k_merge_quads(const uint32_t *__restrict__ seg_off, uint32_t NB,
-                                                    uint4 *__restrict__ seg_sum, uint32_t *__restrict__ heavy,
-                                                    uint32_t *__restrict__ heavy_n, uint32_t heavy_min)
-{
-    using F = typename C::F;
-    using Q = Quad<C>;
-    const Q op(threadIdx.x);
-    const uint32_t stride = gridDim.x * (blockDim.x >> 2);
-    for (uint32_t w = blockIdx.x * (blockDim.x >> 2) + (threadIdx.x >> 5) * 8; w < NB; w += stride) {
-        const uint32_t kb = w + ((threadIdx.x >> 2) & 7);
-        uint32_t s0 = 0, ns = 0;
-        if (kb < NB) {
-            s0 = seg_off[kb];
-            ns = seg_off[kb + 1] - s0;
-            if (ns > heavy_min) {
-                if (op.j == 0)
-                    heavy[atomicAdd(heavy_n, 1u)] = kb;
-                ns = 0;
-            }
-        }
-        const uint32_t most = __reduce_max_sync(Q::ALL, ns);
-        if (most < 2)
-            continue;
-        Fe acc = ns > 1 ? Q::load(seg_sum, s0, op.j) : F::zero();
-        for (uint32_t i = 1; i < most; i++) {
-            const bool take = i < ns;
-            const Fe o = take ? Q::load(seg_sum, s0 + i, op.j) : F::zero();
-            acc = op.template add<false>(acc, o, take);
-        }
-        if (ns > 1)
-            Q::store(seg_sum, s0, op.j, acc);
-    }
-}
-
-template <class C>
 cudaError_t msm_tail(Context &ctx, const BatchPlan &p, const BatchBuffers &b)
 {
     cudaStream_t st = ctx.stream;
-    // a small plan: accumulation and merges on quads
+    // a small plan: accumulation on quads
     const bool small = !p.ba_rounds && !p.part_slice && p.entries_bound <= ACC_QUADS_MAX_ENTRIES;
     // 2. accumulate: a grid of short blocks (up to 32 per SM, several waves), each
     //    thread taking segments at a stride of the grid.  Segments come longest
@@ -1096,18 +1087,12 @@ cudaError_t msm_tail(Context &ctx, const BatchPlan &p, const BatchBuffers &b)
             if (e != cudaSuccess)
                 return e;
         }
-        const int threads = 256;
-        if (small) {
-            const unsigned mb = (unsigned)std::max<uint32_t>(1, std::min<uint32_t>((p.NB + 31) / 32,
-                                                                                   (uint32_t)ctx.sm_count * 8));
-            k_merge_quads<C><<<mb, 128, 0, st>>>(b.seg_off, p.NB, b.seg_sum, b.heavy, b.heavy_n, HEAVY_MIN);
-        } else {
-            k_merge_light<C><<<(p.NB + threads - 1) / threads, threads, 0, st>>>(b.seg_off, p.NB, b.seg_sum,
-                                                                               b.heavy, b.heavy_n, HEAVY_MIN);
-        }
+        const unsigned mb =
+            (unsigned)std::max<uint32_t>(1, std::min<uint32_t>((p.NB + 31) / 32, (uint32_t)ctx.sm_count * 64));
+        k_merge<C><<<mb, 128, 0, st>>>(b.seg_off, p.NB, b.seg_sum, b.heavy, b.heavy_n, HEAVY_MIN);
         HS_LAUNCH_CHECK(ctx);
         if (any_heavy) {
-            k_merge_heavy<C><<<ctx.sm_count, HEAVY_THREADS, 0, st>>>(b.seg_off, b.heavy, b.heavy_n, b.seg_sum);
+            k_merge_heavy<C><<<ctx.sm_count, HEAVY_QUADS * 4, 0, st>>>(b.seg_off, b.heavy, b.heavy_n, b.seg_sum);
             HS_LAUNCH_CHECK(ctx);
         }
     }
