@@ -52,6 +52,12 @@ struct GraphEntry {
 // until hs_context_set_batch_affine sets the curve)
 constexpr uint32_t BA_DEFAULT_ROUNDS[2] = {1, 2};
 constexpr uint64_t BA_DEFAULT_MIN_ENTRIES = uint64_t(1) << 21;
+// by default a plan with nothing beside it takes rounds from here (GB300, us, Helios |
+// Selene: 2^17 points 691 | 920 without, 778 | 1028 with one; 16 x 16384 1051 | 1438
+// and 1105 | 1466; 64 x 8192 1892 | 2628 and 1843 | 2461); the halves of a split MSM
+// and a server's slots fill each other's waits and keep BA_DEFAULT_MIN_ENTRIES (a
+// queue of 96 requests 9.13 ms, 9.42 with this)
+constexpr uint64_t BA_WHOLE_MIN_ENTRIES = uint64_t(7) << 20;
 
 struct Context {
     int device = 0;
@@ -82,6 +88,7 @@ struct Context {
     // both, 5.06 with none on Helios: one curve's memory-bound rounds overlap
     // the other's multiply-bound work.
     uint32_t ba_rounds[2] = {BA_DEFAULT_ROUNDS[0], BA_DEFAULT_ROUNDS[1]};
+    uint64_t ba_whole_min_entries = BA_WHOLE_MIN_ENTRIES;
     uint64_t ba_min_entries[2] = {BA_DEFAULT_MIN_ENTRIES, BA_DEFAULT_MIN_ENTRIES};
     // Until hs_context_set_batch_affine sets a curve, two kinds of plans take
     // their own rounds, because there a curve's MSMs run mostly alone, where
@@ -267,10 +274,14 @@ __device__ __forceinline__ uint32_t find_msm(uint32_t M, uint32_t x, KeyFn key)
     return lo;
 }
 
-int choose_window(const Context &ctx, int curve, size_t n);
+// what a plan's MSMs are: one by itself, one whose bases are decoded from host
+// encodings, a few or many together; fewest_ops bounds a plan's entries
+enum class Widths { alone, decoded, few, many, fewest_ops };
+int choose_window(const Context &ctx, int curve, size_t n, Widths use = Widths::alone);
 // base_rounds >= 0: the batch-affine rounds in place of the curve's setting
 // (a window rule that names rounds still wins)
-BatchPlan make_batch_plan(const Context &ctx, int curve, const size_t *sizes, uint32_t M, int base_rounds = -1);
+BatchPlan make_batch_plan(const Context &ctx, int curve, const size_t *sizes, uint32_t M, int base_rounds = -1,
+                          bool decoded = false);
 // count fixed-base MSMs of n table generators each (window c), scalars back to back
 BatchPlan make_fixed_plan(int curve, size_t n, int c, uint32_t count);
 // M MSMs over rows of one window-multiple table (window c) named by index lists

@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <iterator>
 #include <mutex>
 #include <new>
 
@@ -106,16 +107,48 @@ const CurveOps &curve_ops(int curve) { return curve == HS_SELENE ? selene_ops : 
 // ---------------------------------------------------------------------------
 static constexpr uint32_t SEG_HIST_THREADS = 256;
 
-static int model_window(size_t n)
+// Window widths, measured on GB300 with uniform scalars.  The operation count
+// (fewest_ops_window) does not see what decides between neighbours:
+// - the top window.  Scalars are below 2^255, so the widths that leave it a bit or
+//   two (11, 15, 17) put half of its n entries into one or two buckets, whose
+//   chains outlast everything else: 2^21 Helios points 3.66 ms with c = 16, 5.13
+//   with 17; 2^19 1.30 with 16, 1.49 with 15;
+// - the lists: 2^22 points fill 2^15 buckets a window faster than 2^17 (7.15 ms
+//   with c = 16, 8.62 with 18, 10.05 with 17; Selene 8.73, 10.41, 11.50).
+struct WindowStep {
+    size_t n_max;
+    int c;
+};
+// One MSM by itself is latency-bound up to some 2^16 points: fewer buckets shorten
+// the reduction by more than the added windows cost (Helios | Selene, us: 8192
+// points 335 | 459 with c = 8, 350 | 474 with 10; 16384 378 | 506 with 9, 426 | 559
+// with 11; 2^17 691 | 920 with 14, 718 | 947 with 13; 400000 1131 | 1534 with 14,
+// 1108 | 1512 with 16; 2^25 66.8 | 74.8 ms with 16, 63.4 | 69.4 with 20).  65536 points
+// take 543 | 716 with 13 and 537 | 707 with 14, but both curves' MSMs side by side 843
+// and 892.
+static const WindowStep ALONE_WINDOWS[] = {{10000, 8},  {24000, 9},   {48000, 10},
+                                           {80000, 13}, {350000, 14}, {size_t(1) << 24, 16}};
+// Host encodings: the lists are ready before the bases are decoded, and what is left
+// after that has no sort in it, whose work grows with the number of windows (65521
+// points 679 | 958 with c = 12, 727 | 979 with 14; 2^17 935 | 1380 with 13, 996 | 1402
+// with 14; 200000 1138 | 1665 with 14, 1208 | 1761 with 12).
+static const WindowStep DECODED_WINDOWS[] = {{10000, 8},   {24000, 9},   {40000, 10},          {90000, 12},
+                                             {150000, 13}, {350000, 14}, {size_t(1) << 24, 16}};
+// MSMs of a batch fill the device together, so the operations count (ms: 1024 x 256
+// points 2.60 | 3.66 with c = 6, 2.97 | 4.51 with 8; 4096 x 64 6.23 | 9.31 with 5,
+// 10.0 | 15.8 with 8; 32 x 16384 1.67 | 2.24 with 10, 1.75 | 2.31 with 11; 16 x 65536
+// 2.61 | 3.45 with 12, 2.73 | 3.61 with 13; 2 x 2^19 2.21 | 2.93 with 14, 2.25 | 2.97
+// with 16, 2.37 | 3.13 with 15).
+static const WindowStep BATCH_WINDOWS[] = {{160, 5},    {500, 6},    {1600, 7},   {5000, 8},    {7000, 9},
+                                           {24000, 10}, {90000, 12}, {200000, 13}, {700000, 14}, {size_t(1) << 24, 16}};
+// The narrow widths pay from about this many MSMs, whose 33 x 128 buckets of c = 8
+// the reduction would notice (64 points each, us: 64 MSMs 414 with c = 6, 482 with 8;
+// 8 MSMs 349 with 6, 330 with 8).
+constexpr uint32_t NARROW_MIN_MSMS = 64;
+
+// the fewest additions: W(c) * (n * madd + 2^(c-1) * 2 adds), madd ~ 10 M, add ~ 14 M
+static int fewest_ops_window(size_t n)
 {
-    // cost ~ W(c) * (n * madd + 2^(c-1) * 2 adds), madd ~ 10 M, add ~ 14 M.  A
-    // first guess only: the autotuner (helioselene_gb300.autotune) measures each
-    // size class on the device and installs rules that override it.  On GB300 at
-    // n = 2^20 the measured optimum agrees (c = 16: 16 full windows plus a
-    // carry window that is almost empty).
-    // Below c = 8 the model's work saving does not pay on the GPU: small MSMs are
-    // latency-bound, and c = 8 (32 full windows, the top one with 7 used bits)
-    // measured fastest from 512 to 4096 points on both curves.
     int best = 8;
     double best_cost = 1e300;
     for (int c = 8; c <= 20; c++) {
@@ -129,15 +162,33 @@ static int model_window(size_t n)
     return best;
 }
 
-int choose_window(const Context &ctx, int curve, size_t n)
+int choose_window(const Context &ctx, int curve, size_t n, Widths use)
 {
     int c = 0;
     for (const WindowRule &r : ctx.rules[curve == HS_SELENE ? 1 : 0])
         if (n >= r.n_min && n <= r.n_max)
             c = r.c;
-    if (c < 4 || c > 20)
-        c = model_window(n);
-    return c;
+    if (c >= 4 && c <= 20)
+        return c;
+    const auto step = [n](const WindowStep *s, size_t len) {
+        for (size_t i = 0; i < len; i++)
+            if (n <= s[i].n_max)
+                return s[i].c;
+        return 20;
+    };
+    switch (use) {
+    case Widths::alone:
+        return step(ALONE_WINDOWS, std::size(ALONE_WINDOWS));
+    case Widths::decoded:
+        return step(DECODED_WINDOWS, std::size(DECODED_WINDOWS));
+    case Widths::few:
+        return std::max(8, step(BATCH_WINDOWS, std::size(BATCH_WINDOWS)));
+    case Widths::many:
+        return step(BATCH_WINDOWS, std::size(BATCH_WINDOWS));
+    case Widths::fewest_ops:
+        break;
+    }
+    return fewest_ops_window(n);
 }
 
 // Shared-memory counting sort: MSM m's emitted windows are each cut into
@@ -216,7 +267,22 @@ static uint32_t seg_cap(uint64_t ent, uint64_t nb)
     return (uint32_t)std::min<uint64_t>(big, std::max<uint64_t>(least, ent / 65536));
 }
 
-BatchPlan make_batch_plan(const Context &ctx, int curve, const size_t *sizes, uint32_t M, int base_rounds)
+// The default rounds of a plan (a curve whose rounds were set keeps what was set).
+// A round's launches and inversions are waits: from `least` entries they pay.  A
+// second round pays for one MSM in long lists of many entries (Selene on GB300, us:
+// 2^21 points 4657 with one round, 4525 with two; 2^19 1762 and 1853; 2^18 1280 and
+// 1455); the MSMs of a batch, mostly beside the other curve's, keep theirs.
+constexpr uint64_t BA_TWO_MIN_ENTRIES = uint64_t(1) << 23;
+
+static uint32_t default_rounds(const BatchPlan &p, uint32_t rounds, uint64_t least)
+{
+    if (p.entries_bound < least)
+        return 0;
+    return p.M > 1 || p.entries_bound >= BA_TWO_MIN_ENTRIES ? rounds : std::min<uint32_t>(rounds, 1);
+}
+
+BatchPlan make_batch_plan(const Context &ctx, int curve, const size_t *sizes, uint32_t M, int base_rounds,
+                          bool decoded)
 {
     BatchPlan p;
     p.curve = curve;
@@ -224,10 +290,22 @@ BatchPlan make_batch_plan(const Context &ctx, int curve, const size_t *sizes, ui
     p.msms.resize(M);
     uint64_t nb_all = 0;
     std::vector<int> cs(M);
+    const Widths use = M >= NARROW_MIN_MSMS ? Widths::many
+                       : M > 1              ? Widths::few
+                       : decoded            ? Widths::decoded
+                                            : Widths::alone;
+    uint64_t ent_all = 0;
     for (uint32_t i = 0; i < M; i++) {
-        cs[i] = choose_window(ctx, curve, sizes[i] ? sizes[i] : 1);
-        nb_all += (uint64_t)((257 + cs[i] - 1) / cs[i]) << (cs[i] - 1);
+        cs[i] = choose_window(ctx, curve, sizes[i] ? sizes[i] : 1, use);
+        ent_all += (uint64_t)sizes[i] * ((257 + cs[i] - 1) / cs[i]);
     }
+    // at the limit of what one launch sequence indexes, the windows of fewest operations
+    // (and so fewest entries) decide whether a batch is taken
+    if (ent_all >= 0x80000000ull)
+        for (uint32_t i = 0; i < M; i++)
+            cs[i] = choose_window(ctx, curve, sizes[i] ? sizes[i] : 1, Widths::fewest_ops);
+    for (uint32_t i = 0; i < M; i++)
+        nb_all += (uint64_t)((257 + cs[i] - 1) / cs[i]) << (cs[i] - 1);
     const uint32_t gsz = group_size(nb_all);
     uint64_t pt = 0, nb = 0, g = 0, ws = 0, ent = 0;
     for (uint32_t i = 0; i < M; i++) {
@@ -274,6 +352,8 @@ BatchPlan make_batch_plan(const Context &ctx, int curve, const size_t *sizes, ui
     // the plan's entries when that rule names some, else the curve's setting
     const auto &rules = ctx.rules[curve == HS_SELENE ? 1 : 0];
     int rounds = base_rounds >= 0 ? base_rounds : (int)ctx.ba_rounds[curve == HS_SELENE];
+    if (!ctx.ba_set[curve == HS_SELENE])
+        rounds = (int)default_rounds(p, (uint32_t)rounds, ctx.ba_whole_min_entries);
     if (!rules.empty()) {
         std::vector<uint64_t> by_rule(rules.size(), 0);
         for (uint32_t i = 0; i < M; i++) {
@@ -1827,8 +1907,9 @@ static SplitPlan make_split(const Context &ctx, int curve, size_t n, int base_ro
     SplitPlan sp{make_window_plan(curve, n, c, h, W - h), make_window_plan(curve, n, c, 0, h)};
     const int k = curve == HS_SELENE;
     const uint32_t rounds = base_rounds >= 0 ? (uint32_t)base_rounds : ctx.ba_rounds[k];
-    plan_batch_affine(sp.hi, rounds, ctx.ba_min_entries[k]);
-    plan_batch_affine(sp.lo, rounds, ctx.ba_min_entries[k]);
+    const uint64_t least = BA_DEFAULT_MIN_ENTRIES;  // the rounds' waits are filled by the other half
+    plan_batch_affine(sp.hi, ctx.ba_set[k] ? rounds : default_rounds(sp.hi, rounds, least), ctx.ba_min_entries[k]);
+    plan_batch_affine(sp.lo, ctx.ba_set[k] ? rounds : default_rounds(sp.lo, rounds, least), ctx.ba_min_entries[k]);
     return sp;
 }
 
@@ -2229,7 +2310,7 @@ static int msm_host(Context &ctx, int curve, const uint8_t *lead_scalar, const v
         s = make_split(ctx, curve, total, base_rounds);
     else {
         const size_t sizes[1] = {total};
-        p = make_batch_plan(ctx, curve, sizes, 1, base_rounds);
+        p = make_batch_plan(ctx, curve, sizes, 1, base_rounds, point_fmt == HS_FMT_COMPRESSED);
     }
     // Bases spanning several counting-sort slices arrive in two parts, split at a
     // slice boundary: the entries of a bucket come in slice order, so each part's
@@ -3044,12 +3125,22 @@ int hs_measure_imad_rates(hs_context *h, double rates[4])
 }
 
 // ---- fixed-base commitments ----
+// One reduction window for all windows of the table: the operation count, W(c) * n
+// * madd + 2^(c-1) * 2 adds, decides while it asks for at most 16 bits.  Above that
+// 17 to 19 bits lose to 16, whose buckets the sort fills faster and whose last full
+// window is as even as the others (8 commitments over 2^18 generators on GB300, ms,
+// Helios | Selene: 3.65 | 4.47 with 16, 4.07 | 5.18 with 18; 2^19: 6.77 | 8.69 with
+// 16, 7.73 | 9.70 with 18), and 20 bits, 13 windows for 16, pay from some 2^20
+// generators (6.83 | 9.28 at 2^19; 2^20: 13.4 | 17.5 with 16, 12.4 | 16.5 with 20).
+constexpr size_t FIXED_WIDE_MIN = 800000;
+
 static int fixed_window(size_t n)
 {
-    // one reduction window: cost ~ W(c) * n * madd + 2^(c-1) * 2 adds
+    if (n >= FIXED_WIDE_MIN)
+        return 20;
     int best = 8;
     double best_cost = 1e300;
-    for (int c = 6; c <= 20; c++) {
+    for (int c = 6; c <= 16; c++) {
         const double W = (257 + c - 1) / c;
         const double cost = W * 10.0 * (double)n + 28.0 * (double)(1u << (c - 1));
         if (cost < best_cost) {

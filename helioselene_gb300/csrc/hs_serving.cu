@@ -121,13 +121,14 @@ static bool table_form(const Server &S, const hs_request &q)
 }
 
 // (point, window) entries of a request under the slots' window rules, or the
-// pool table's windows
+// pool table's windows: what a batch of requests is bounded by (a plan whose own
+// widths exceed the bound takes these)
 static uint64_t request_entries(const Server &S, const hs_request &q)
 {
     const size_t n = q.n_pool + q.n_fresh;
     if (table_form(S, q))
         return (uint64_t)n * S.pools[q.curve].W;
-    const int c = choose_window(S.slots[0]->ctx, q.curve, n ? n : 1);
+    const int c = choose_window(S.slots[0]->ctx, q.curve, n ? n : 1, Widths::fewest_ops);
     return (uint64_t)n * (uint64_t)((257 + c - 1) / c);
 }
 
@@ -534,6 +535,7 @@ int hs_server_create(hs_server **out, const hs_server_config *cfg)
         sl->ctx.device = S.cfg.device;
         sl->ctx.sm_count = sms;
         sl->ctx.pageable_access = pageable == 1;
+        sl->ctx.ba_whole_min_entries = BA_DEFAULT_MIN_ENTRIES;
         sl->ctx.use_graphs = false;  // request shapes rarely repeat
         if (cudaStreamCreateWithFlags(&sl->ctx.stream, cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&sl->done, cudaEventDisableTiming) != cudaSuccess) {
