@@ -17,6 +17,8 @@
 //      per-window doublings, :285-289) on one warp, result as canonical Jacobian.
 #pragma once
 
+#include <cooperative_groups.h>
+
 #include "hs_curve.cuh"
 #include "hs_internal.h"
 #include "hs_lane.cuh"
@@ -750,6 +752,8 @@ __global__ void __launch_bounds__(RED_QUADS * 4) k_window_sum(const uint4 *__res
 // ---------------------------------------------------------------------------
 // 5. window combination (Horner) -> canonical Jacobian
 // ---------------------------------------------------------------------------
+constexpr uint32_t COMBINE_MAX_GROUPS = 8;  // a cluster's blocks
+
 template <class C>
 __device__ void store_jacobian_canon(uint32_t *out, const Xyzz &p)
 {
@@ -768,29 +772,40 @@ __device__ void store_jacobian_canon(uint32_t *out, const Xyzz &p)
     }
 }
 
-// one block of four warps per MSM of the batch (hs_lane.cuh)
+// One block of four warps per group of an MSM's windows (hs_lane.cuh), the G groups of
+// an MSM a cluster.  The chain's doublings can't be shortened, but its additions can:
+// block r of the cluster sums the r-th group from the top by itself, in the time that
+// block 0 takes for the top group, and hands the sum to block 0, whose chain goes on
+// with one addition per group instead of one per window.  Blocks of a cluster with
+// no windows left hand over nothing.
 template <class C>
 __global__ void __launch_bounds__(128, 1) k_combine(const uint4 *__restrict__ S, const MsmDesc *__restrict__ desc,
-                                                   uint32_t *__restrict__ out)
+                                                   uint32_t *__restrict__ out, uint32_t G)
 {
     using F = typename C::F;
     using LF = LaneField<F>;
     __shared__ LaneSlot sl[LNSLOTS];
     __shared__ alignas(16) uint32_t ad[LN_MAX_WINDOWS][48];  // the window sums' limbs, coordinate by coordinate
     __shared__ uint32_t nonzero[LN_MAX_WINDOWS];
-    const MsmDesc d = desc[blockIdx.x];
-    const uint4 *Sm = S + 8 * (size_t)d.win_base;
+    __shared__ alignas(16) uint32_t gsum[COMBINE_MAX_GROUPS][48];  // block 0: the groups' sums
+    __shared__ uint32_t gnonzero[COMBINE_MAX_GROUPS];
+    const uint32_t mi = blockIdx.x / G, rank = blockIdx.x - mi * G;
+    const MsmDesc d = desc[mi];
     if (d.Wr == 1 && d.shift == 0) {  // one window (fixed base): nothing to combine
-        if (threadIdx.x == 0)
-            store_jacobian_canon<C>(out + 24 * (size_t)blockIdx.x, load_xyzz(Sm));
+        if (rank == 0 && threadIdx.x == 0)
+            store_jacobian_canon<C>(out + 24 * (size_t)mi, load_xyzz(S + 8 * (size_t)d.win_base));
         return;
     }
+    const uint32_t per = (d.Wr + G - 1) / G;
+    const uint32_t top = d.Wr > rank * per ? d.Wr - rank * per : 0;  // this block's windows: [low, top)
+    const uint32_t low = top > per ? top - per : 0;
+    const uint4 *Sm = S + 8 * ((size_t)d.win_base + low);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     LaneHorner<C> h(sl, lane, warp);
     for (uint32_t i = threadIdx.x; i < sizeof(sl) / 4; i += blockDim.x)
         reinterpret_cast<uint32_t *>(sl)[i] = 0;
     // every window sum's limbs up front (the chain then waits for no global load)
-    for (uint32_t i = warp; i < 4 * d.Wr; i += 4) {
+    for (uint32_t i = warp; i < 4 * (top - low); i += 4) {
         const uint32_t k = i >> 2, c = i & 3;
         const Fe v = load_fe(Sm + 8 * (size_t)k + 2 * c);
         const uint32_t limb = LF::from_fe(v, lane);
@@ -801,23 +816,49 @@ __global__ void __launch_bounds__(128, 1) k_combine(const uint4 *__restrict__ S,
     }
     __syncthreads();
     bool ident = true;
-    for (int k = (int)d.Wr - 1; k >= 0; k--) {
-        if (!ident && k < (int)d.Wr - 1)
-            for (uint32_t i = 0; i < d.c; i++)
+    const auto step = [&](uint32_t doublings, const uint32_t *a, uint32_t nz) {
+        if (!ident)
+            for (uint32_t i = 0; i < doublings; i++)
                 h.dbl();
-        if (!nonzero[k])
-            continue;
+        if (!nz)
+            return;
         if (ident) {
-            h.take(ad[k]);
+            h.take(a);
             ident = false;
-            continue;
+            return;
         }
-        const int r = h.add(ad[k]);
+        const int r = h.add(a);
         if (r == 1) {  // equal operands: double
             __syncthreads();
             h.dbl();
         } else if (r == 2) {  // they cancel
             ident = true;
+        }
+    };
+    for (uint32_t k = top - low; k-- > 0;)
+        step(d.c, ad[k], nonzero[k]);
+    if (G > 1) {
+        namespace cg = cooperative_groups;
+        cg::cluster_group cluster = cg::this_cluster();
+        cluster.sync();  // block 0 runs and its shared memory may be written
+        if (rank) {
+            __syncthreads();
+            // coordinate `warp` in exact limbs, as a window sum's
+            const LaneSlot &co = sl[warp == 0 ? LX0 + h.x : warp == 1 ? LY : warp == 2 ? LZZ : LZZZ];
+            const uint32_t limb = LF::from_fe(LF::to_fe(warp == 3 ? h.f.own_w(co) : h.f.own(co)), lane);
+            uint32_t *dst = cluster.map_shared_rank(&gsum[0][0], 0);
+            if (lane < 12)
+                dst[48 * rank + 12 * warp + lane] = limb;
+            if (threadIdx.x == 0)
+                *cluster.map_shared_rank(&gnonzero[rank], 0) = ident ? 0u : 1u;
+        }
+        cluster.sync();
+        if (rank)
+            return;
+        for (uint32_t r = 1, t = low; t; r++) {  // group r: windows [t - size, t)
+            const uint32_t size = t < per ? t : per;
+            step(d.c * size, gsum[r], gnonzero[r]);
+            t -= size;
         }
     }
     if (!ident)
@@ -833,8 +874,40 @@ __global__ void __launch_bounds__(128, 1) k_combine(const uint4 *__restrict__ S,
             t.ZZZ = LF::to_fe(h.f.own_w(sl[LZZZ]));
         }
         if (lane == 0)
-            store_jacobian_canon<C>(out + 24 * (size_t)blockIdx.x, t);
+            store_jacobian_canon<C>(out + 24 * (size_t)mi, t);
     }
+}
+
+// Groups of windows per MSM, while every block has an SM to itself: two on one slow each
+// other's chains by more than the additions were worth (GB300, 64-point MSMs, Helios |
+// Selene, us: 19 of them 369 | 499 without groups, 360 | 488 with; 38 of them 423 |
+// 562 and 426 | 600).  With them one MSM of 16 points from host memory takes 267 us
+// instead of 289, 65521 encodings 945 instead of 962.
+static uint32_t combine_groups(const BatchPlan &p, int sm_count)
+{
+    uint32_t wr = 1;
+    for (const MsmDesc &d : p.msms)
+        wr = std::max(wr, d.Wr);
+    const uint32_t G = wr >= 28 ? COMBINE_MAX_GROUPS : wr >= 16 ? 5 : wr >= 8 ? 3 : 1;
+    return (uint64_t)p.M * G <= (uint64_t)sm_count ? G : 1;
+}
+
+template <class C>
+static cudaError_t launch_combine(Context &ctx, const BatchPlan &p, const BatchBuffers &b, cudaStream_t st)
+{
+    const uint32_t G = combine_groups(p, ctx.sm_count);
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = G;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(p.M * G);
+    cfg.blockDim = dim3(128);
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_combine<C>, (const uint4 *)b.redS, (const MsmDesc *)b.desc,
+                              (uint32_t *)b.out_jac, G);
 }
 
 // Window sums of a plan of few windows of at most WQ_MAX_B buckets, where the
@@ -1128,8 +1201,10 @@ cudaError_t msm_tail(Context &ctx, const BatchPlan &p, const BatchBuffers &b)
             HS_LAUNCH_CHECK(ctx);
         }
     }
-    // 5. Horner over windows, one block of four warps per MSM
-    k_combine<C><<<p.M, 128, 0, st>>>(b.redS, b.desc, b.out_jac);
+    // 5. Horner over windows, a cluster of blocks of four warps per MSM
+    const cudaError_t e = launch_combine<C>(ctx, p, b, st);
+    if (e != cudaSuccess)
+        return e;
     HS_LAUNCH_CHECK(ctx);
     return cudaSuccess;
 }
