@@ -164,6 +164,17 @@ constexpr uint32_t SMALL_SORT_MAX_NB = 8192;
 constexpr uint64_t SMALL_SORT_MAX_ENTRIES = 98304;
 constexpr size_t SMALL_SORT_SMEM = (2 * (size_t)SMALL_SORT_MAX_NB + 160) * 4;
 
+constexpr uint32_t BA_MAX_ROUNDS = 3;
+constexpr uint32_t PAD_ENTRY = 0xffffffffu;  // an entry that adds nothing (batch-affine lists)
+
+// the block sort of a batch of small fixed-base MSMs (k_recode_block): an MSM's
+// buckets and entries, the least MSMs
+constexpr uint32_t BLOCK_SORT_MAX_B = 4096;
+constexpr uint32_t BLOCK_SORT_ENTRIES = 20480;
+constexpr uint32_t BLOCK_SORT_MIN_MSMS = 128;
+// buckets, entries and the most padding (2^BA_MAX_ROUNDS - 1 a bucket)
+constexpr size_t BLOCK_SORT_SMEM = (((size_t)BLOCK_SORT_MAX_B << BA_MAX_ROUNDS) + BLOCK_SORT_ENTRIES) * 4;
+
 // A run of MSMs sharing one window width (one templated recode launch).
 struct WindowClass {
     int c;
@@ -188,6 +199,8 @@ struct BatchPlan {
     uint32_t sort_blocks = 0;   // counting-sort blocks (shared-memory path)
     uint64_t cnt_len = 0;       // per-block bucket counts (shared-memory path)
     bool global_sort = false;   // keep the global-atomic sort (no digit and count buffers)
+    bool block_sort = false;    // the block sort of small fixed-base MSMs instead of it
+    uint32_t block_sort_entries = 0, block_sort_threads = 0;  // the largest block's
     bool smem_sort() const { return !global_sort && max_B <= SORT_SMEM_MAX_B; }
     // One MSM whose buckets and entries a single block sorts in shared memory
     // (k_sort_small): one launch for the recode, the sort and the segments instead of
@@ -224,7 +237,6 @@ struct BatchPlan {
 // rounds at most
 constexpr uint32_t BA_PLAN_K = 32;
 constexpr uint32_t BA_PLAN_BT = 128;
-constexpr uint32_t BA_MAX_ROUNDS = 3;
 
 // Device buffers of one batch (carved from the arena).
 struct BatchBuffers {

@@ -170,7 +170,6 @@ __global__ void __launch_bounds__(128, 4) k_accumulate(const uint4 *__restrict__
 // sums by k_accumulate_level.
 constexpr int BA_K = (int)BA_PLAN_K;    // outputs per thread
 constexpr int BA_BT = (int)BA_PLAN_BT;  // threads per block
-constexpr uint32_t PAD_ENTRY = 0xffffffffu;
 
 enum BaKind : int { BA_ADD, BA_DBL, BA_COPY_A, BA_COPY_B, BA_ZERO };
 
