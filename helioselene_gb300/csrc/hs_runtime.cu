@@ -662,33 +662,51 @@ __device__ __forceinline__ uint32_t window_bits(const uint32_t s[8], int k)
 template <int CB, bool SCATTER>
 __device__ __forceinline__ void recode_one(const uint32_t s[8], uint32_t pbase, uint32_t pstep, uint32_t wstep,
                                            uint32_t bucket_base, uint32_t w_lo, uint32_t w_cnt,
-                                           uint32_t *__restrict__ counts, const uint32_t *__restrict__ offsets,
-                                           uint32_t *__restrict__ sorted)
+                                           uint32_t *__restrict__ cursor, uint32_t *__restrict__ sorted)
 {
-    constexpr int W = (257 + CB - 1) / CB;
+    constexpr int W = (257 + CB - 1) / CB, U = SCATTER ? 4 : 1;
     constexpr uint32_t B = 1u << (CB - 1);
     uint32_t carry = 0;
 #pragma unroll
-    for (int k = 0; k < W; k++) {
-        const uint32_t v = window_bits<CB>(s, k) + carry;
-        uint32_t mag;
-        bool neg = false;
-        if (k < W - 1 && v >= B) {
-            mag = (1u << CB) - v;  // digit v - 2^c < 0
-            neg = mag != 0;
-            carry = 1;
-        } else {
-            mag = v;
-            carry = 0;
-        }
-        if (mag != 0 && (uint32_t)k - w_lo < w_cnt) {
-            const uint32_t kb = bucket_base + ((uint32_t)k - w_lo) * wstep + mag - 1u;
-            if (!SCATTER) {
-                atomicAdd(counts + kb, 1u);
+    for (int k0 = 0; k0 < W; k0 += U) {
+        // the cursors of U digits are fetched together, then their entries stored
+        uint32_t kb[U], val[U], pos[U];
+        bool emit[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int k = k0 + u;
+            emit[u] = false;
+            if (k >= W)
+                continue;
+            const uint32_t v = window_bits<CB>(s, k) + carry;
+            uint32_t mag;
+            bool neg = false;
+            if (k < W - 1 && v >= B) {
+                mag = (1u << CB) - v;  // digit v - 2^c < 0
+                neg = mag != 0;
+                carry = 1;
             } else {
-                const uint32_t pos = offsets[kb] + atomicAdd(counts + kb, 1u);
-                sorted[pos] = (pbase + (uint32_t)k * pstep) | (neg ? 0x80000000u : 0u);
+                mag = v;
+                carry = 0;
             }
+            emit[u] = mag != 0 && (uint32_t)k - w_lo < w_cnt;
+            kb[u] = bucket_base + ((uint32_t)k - w_lo) * wstep + mag - 1u;
+            val[u] = (pbase + (uint32_t)k * pstep) | (neg ? 0x80000000u : 0u);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (!emit[u])
+                continue;
+            if (SCATTER)
+                pos[u] = atomicAdd(cursor + kb[u], 1u);
+            else
+                atomicAdd(cursor + kb[u], 1u);
+        }
+        if (SCATTER) {
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (emit[u])
+                    sorted[pos[u]] = val[u];
         }
     }
 }
@@ -702,8 +720,8 @@ __device__ __forceinline__ uint32_t table_gen(const MsmDesc &d, const uint32_t *
 
 template <bool SCATTER>
 __global__ void k_recode(const uint4 *__restrict__ scalars, uint32_t n_total, const MsmDesc *__restrict__ desc,
-                         uint32_t M, uint32_t *__restrict__ counts, const uint32_t *__restrict__ offsets,
-                         uint32_t *__restrict__ sorted, const uint32_t *__restrict__ pt_idx)
+                         uint32_t M, uint32_t *__restrict__ cursor, uint32_t *__restrict__ sorted,
+                         const uint32_t *__restrict__ pt_idx)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_total)
@@ -720,7 +738,7 @@ __global__ void k_recode(const uint4 *__restrict__ scalars, uint32_t n_total, co
     switch (c) {
 #define HS_CASE(v)                                                       \
     case v:                                                              \
-        recode_one<v, SCATTER>(s, pbase, pstep, wstep, base, w_lo, w_cnt, counts, offsets, sorted); \
+        recode_one<v, SCATTER>(s, pbase, pstep, wstep, base, w_lo, w_cnt, cursor, sorted);         \
         break;
         HS_CASE(4)
         HS_CASE(5)
@@ -930,7 +948,7 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_scatter(const uint32_t *_
 {
     extern __shared__ uint32_t slot[];
     const SortBlock sb = sort_block(desc, M, blockIdx.x);
-    const MsmDesc &d = desc[sb.m];
+    const MsmDesc d = desc[sb.m];
     const uint64_t Bm = d.fixed ? d.B : (uint64_t)d.w_cnt * d.B;
     const uint32_t *row = cnt + d.cnt_base + (uint64_t)sb.q * Bm + sb.col;
     for (uint32_t j = threadIdx.x; j < d.B; j += blockDim.x)
@@ -938,29 +956,26 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_scatter(const uint32_t *_
     __syncthreads();
     const uint32_t *dg = digits + d.dig_base + (size_t)(sb.k_abs - d.w_lo) * d.n;
     const uint32_t step = blockDim.x;
-    uint32_t i = sb.lo + threadIdx.x;
-    for (; i + 3 * step < sb.hi; i += 4 * step) {
-        uint32_t dv[4];
+    // U digits, then their cursors, then their entries: the three waits are shared
+    constexpr int U = 8;
+    for (uint32_t i0 = sb.lo + threadIdx.x; i0 < sb.hi; i0 += U * step) {
+        uint32_t dv[U], pos[U];
 #pragma unroll
-        for (int u = 0; u < 4; u++)
-            dv[u] = __ldg(dg + (i + u * step - d.pt_off));
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const uint32_t mag = dv[u] & 0x7fffffffu;
-            if (mag) {
-                const uint32_t ii = i + u * step;
-                const uint32_t pos = atomicAdd(slot + mag - 1, 1u);
-                const uint32_t v = d.fixed ? table_gen(d, pt_idx, ii) * d.W + sb.k_abs : ii;
-                sorted[pos] = v | (dv[u] & 0x80000000u);
-            }
+        for (int u = 0; u < U; u++) {
+            const uint32_t i = i0 + u * step;
+            dv[u] = i < sb.hi ? __ldg(dg + (i - d.pt_off)) : 0u;
         }
-    }
-    for (; i < sb.hi; i += step) {
-        const uint32_t dv = __ldg(dg + (i - d.pt_off)), mag = dv & 0x7fffffffu;
-        if (mag) {
-            const uint32_t pos = atomicAdd(slot + mag - 1, 1u);
-            const uint32_t v = d.fixed ? table_gen(d, pt_idx, i) * d.W + sb.k_abs : i;
-            sorted[pos] = v | (dv & 0x80000000u);
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (dv[u] & 0x7fffffffu)
+                pos[u] = atomicAdd(slot + (dv[u] & 0x7fffffffu) - 1, 1u);
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (dv[u] & 0x7fffffffu) {
+                const uint32_t i = i0 + u * step;
+                const uint32_t v = d.fixed ? table_gen(d, pt_idx, i) * d.W + sb.k_abs : i;
+                sorted[pos[u]] = v | (dv[u] & 0x80000000u);
+            }
         }
     }
 }
@@ -1487,18 +1502,17 @@ cudaError_t launch_sort(Context &ctx, const BatchPlan &p, const BatchBuffers &b)
     } else {
         const unsigned rblocks = (p.n_total + 255) / 256;
         if (p.n_total) {
-            k_recode<false><<<rblocks, 256, 0, st>>>(sc, p.n_total, b.desc, p.M, b.counts, b.offsets, b.sorted,
-                                                      b.pt_idx);
+            k_recode<false><<<rblocks, 256, 0, st>>>(sc, p.n_total, b.desc, p.M, b.counts, b.sorted, b.pt_idx);
             HS_LAUNCH_CHECK(ctx);
         }
         if ((e = launch_scan(ctx, b.counts, p.NB, seg_L, b.offsets, b.seg_off, b.scan_tmp, nullptr, pad)) !=
             cudaSuccess)
             return e;
-        if ((e = cudaMemsetAsync(b.counts, 0, (size_t)(p.NB + 1) * 4, st)) != cudaSuccess)
+        // the counts become the buckets' cursors
+        if ((e = cudaMemcpyAsync(b.counts, b.offsets, (size_t)p.NB * 4, cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
             return e;
         if (p.n_total) {
-            k_recode<true><<<rblocks, 256, 0, st>>>(sc, p.n_total, b.desc, p.M, b.counts, b.offsets, b.sorted,
-                                                     b.pt_idx);
+            k_recode<true><<<rblocks, 256, 0, st>>>(sc, p.n_total, b.desc, p.M, b.counts, b.sorted, b.pt_idx);
             HS_LAUNCH_CHECK(ctx);
         }
     }
