@@ -748,6 +748,60 @@ __global__ void __launch_bounds__(RED_QUADS * 4) k_window_sum(const uint4 *__res
         Q::store(S, s, op.j, v);
 }
 
+// Level 2 of a plan of many windows: one quad per window, which runs the window's T
+// groups down in turn,
+//     sum_t acc_t + m0 sum_t t run_t,   sum_t t run_t = sum_{t >= 1} sum_{h >= t} run_h.
+// Three additions per group and no scan, tree or barrier: where the windows fill the
+// device, this does with some 3 steps of a whole warp per window of 8 groups what
+// k_window_chunks' block per window did with 13.  Bound by the multiplier.  GB300: 4 x
+// 256 verification batches 2.10 -> 1.79 ms, 1024 MSMs of 64 to 65536 points 28.4 ->
+// 27.2 ms, 8192 commitments to 228 generators 7.02 -> 6.64 ms, 4096 x 64 points 6.33 |
+// 9.73 -> 4.28 | 6.98 ms (Helios | Selene).
+// The chain of 3 T additions has to be outweighed by the windows there are, 64 per group
+// (GB300, us, Helios: 64 x 512 points, 2752 windows of 8 groups, 527 without and 512
+// with; 100 x 2048, 3300 of 16, 1147 and 1098; 40 x 2048, 1320 of 16, 644 and 746;
+// 100 x 8192, 2600 of 64, 2658 and 2803).
+constexpr int WS_QUADS = 32;
+constexpr uint32_t WS_MIN_WINDOWS = 2048;
+constexpr uint32_t WS_WINDOWS_PER_GROUP = 64;
+
+template <class C>
+__global__ void __launch_bounds__(WS_QUADS * 4) k_window_serial(const uint4 *__restrict__ in,
+                                                               const MsmDesc *__restrict__ desc, uint32_t M,
+                                                               uint32_t WS, uint4 *__restrict__ S)
+{
+    using F = typename C::F;
+    using Q = Quad<C>;
+    const Q op(threadIdx.x);
+    const uint32_t s = blockIdx.x * WS_QUADS + (threadIdx.x >> 2);
+    uint32_t T = 0, doublings = 0;
+    size_t lo = 0;
+    if (s < WS) {
+        const MsmDesc &d = desc[find_msm(M, s, [&](uint32_t k) { return desc[k].win_base; })];
+        T = d.T;
+        doublings = d.log2m0;
+        lo = (size_t)d.group_base + (size_t)(s - d.win_base) * T;
+    }
+    const uint32_t tmax = __reduce_max_sync(Q::ALL, T), dmax = __reduce_max_sync(Q::ALL, doublings);
+    Fe a = F::zero(), r = F::zero(), w = F::zero();
+    for (uint32_t t = tmax; t-- > 0;) {
+        const bool take = t < T;
+        const Fe ta = take ? Q::load(in, 2 * (lo + t), op.j) : F::zero();
+        const Fe tr = take ? Q::load(in, 2 * (lo + t) + 1, op.j) : F::zero();
+        a = op.template add<false>(a, ta, take);
+        r = op.template add<false>(r, tr, take);
+        if (t > 0)
+            w = op.template add<false>(w, r, take);
+    }
+    for (uint32_t m = 0; m < dmax; m++) {
+        const Fe x = op.dbl(w);
+        w = Q::sel(m < doublings, x, w);
+    }
+    w = op.template add<false>(w, a, true);
+    if (s < WS)
+        Q::store(S, s, op.j, w);
+}
+
 // ---------------------------------------------------------------------------
 // 5. window combination (Horner) -> canonical Jacobian
 // ---------------------------------------------------------------------------
@@ -905,8 +959,12 @@ static cudaError_t launch_combine(Context &ctx, const BatchPlan &p, const BatchB
     cfg.stream = st;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_combine<C>, (const uint4 *)b.redS, (const MsmDesc *)b.desc,
-                              (uint32_t *)b.out_jac, G);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_combine<C>, (const uint4 *)b.redS, (const MsmDesc *)b.desc,
+                                             (uint32_t *)b.out_jac, G);
+    if (e != cudaSuccess)
+        return e;
+    HS_LAUNCH_CHECK(ctx);
+    return cudaSuccess;
 }
 
 // Window sums of a plan of few windows of at most WQ_MAX_B buckets, where the
@@ -1179,6 +1237,12 @@ cudaError_t msm_tail(Context &ctx, const BatchPlan &p, const BatchBuffers &b)
         k_reduce_groups<C><<<(p.G + threads - 1) / threads, threads, 0, st>>>(b.seg_off, b.seg_sum, b.desc, p.M,
                                                                             p.G, b.redA);
         HS_LAUNCH_CHECK(ctx);
+        if (p.WS >= std::max(WS_MIN_WINDOWS, WS_WINDOWS_PER_GROUP * p.max_T)) {
+            k_window_serial<C><<<(p.WS + WS_QUADS - 1) / WS_QUADS, WS_QUADS * 4, 0, st>>>(b.redA, b.desc, p.M, p.WS,
+                                                                                        b.redS);
+            HS_LAUNCH_CHECK(ctx);
+            return launch_combine<C>(ctx, p, b, st);
+        }
         // A plan of few chunks (one or a few MSMs) is latency-bound, and so are
         // windows of at most 16 groups: one thread per group up to
         // RED_CHUNK_THREADS groups.  Many chunks of more groups (a batch of larger
@@ -1201,11 +1265,7 @@ cudaError_t msm_tail(Context &ctx, const BatchPlan &p, const BatchBuffers &b)
         }
     }
     // 5. Horner over windows, a cluster of blocks of four warps per MSM
-    const cudaError_t e = launch_combine<C>(ctx, p, b, st);
-    if (e != cudaSuccess)
-        return e;
-    HS_LAUNCH_CHECK(ctx);
-    return cudaSuccess;
+    return launch_combine<C>(ctx, p, b, st);
 }
 
 // ---------------------------------------------------------------------------

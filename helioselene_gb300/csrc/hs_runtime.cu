@@ -262,13 +262,13 @@ static void plan_chunks(BatchPlan &p)
 // Buckets per level-1 group for a plan of nb buckets.  A group is one thread's
 // chain of 2 m0 additions and the groups are level 1's parallelism: 8 for one
 // large MSM, fewer for small plans (latency-bound, so shorter chains on more
-// threads win), more once there are millions of buckets, so that level 2 --
-// latency-bound, a scan per window -- has fewer groups to combine.
+// threads win), more for batches of many buckets, whose level 2 has fewer groups to
+// combine then (GB300: 128 x 8192 points 3250 us with 8, 3212 with 16).
 static uint32_t group_size(uint64_t nb)
 {
     if (nb >= (1ull << 22))
         return 4 * RED_GROUP;
-    if (nb >= (1ull << 21))
+    if (nb >= (1ull << 19))
         return 2 * RED_GROUP;
     if (nb >= (1ull << 18))
         return RED_GROUP;
