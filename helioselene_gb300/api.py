@@ -110,8 +110,8 @@ class Context:
 
     def default_batch_affine(self) -> None:
         """the library's default accumulation forms: one batch-affine round on Helios and two
-        on Selene, except fixed-base commitments and single MSMs from host buffers, which
-        take none on Helios and one on Selene"""
+        on Selene, except fixed-base commitments (none and two) and single MSMs from host
+        buffers (none and one)"""
         self.set_batch_affine(-1)
 
     # -- instrumentation --

@@ -80,25 +80,19 @@ struct Context {
     bool capturing_host = false;
     size_t split_min = size_t(1) << 18;  // single MSMs this large run as two window halves (0: never)
     // Batch-affine accumulation per curve: rounds (0: off) for plans of at
-    // least ba_min_entries entries.  Measured at n = 2^20 on GB300
-    // (accumulation per MSM, ms): Selene 2.54 -> 2.29 with one round, 2.27
-    // with two; Helios 1.55 -> 1.56 with one.  For a Helios and a Selene MSM
-    // side by side on two streams, back to back (the throughput form): 4.78
-    // ms per pair with one round on Helios and two on Selene, 5.07 with one on
-    // both, 5.06 with none on Helios: one curve's memory-bound rounds overlap
-    // the other's multiply-bound work.
+    // least ba_min_entries entries.  One MSM of 2^20 points on GB300 with none, one and
+    // two rounds, us: Helios 2111, 2038, 2085; Selene 2919, 2702, 2727; of 2^21: 3729,
+    // 3617, 3604 and 5160, 4657, 4525.  Side by side the second round on Selene pays
+    // sooner: one curve's memory-bound rounds overlap the other's multiply-bound work.
     uint32_t ba_rounds[2] = {BA_DEFAULT_ROUNDS[0], BA_DEFAULT_ROUNDS[1]};
     uint64_t ba_whole_min_entries = BA_WHOLE_MIN_ENTRIES;
     uint64_t ba_min_entries[2] = {BA_DEFAULT_MIN_ENTRIES, BA_DEFAULT_MIN_ENTRIES};
     // Until hs_context_set_batch_affine sets a curve, two kinds of plans take
     // their own rounds, because there a curve's MSMs run mostly alone, where
     // the round pays on Selene only:
-    // - fixed-base commitments (4096 over 2^20 generators on GB300: Helios 617
-    //   commitments/s without a round, 568 with; Selene 397 without, 427 with);
-    // - single MSMs from host buffers, whose accumulation is pipelined with
-    //   the link (a Helios and a Selene call of 2^20 points from two host
-    //   threads: 6.06 ms per pair with one round on both, 5.91 ms without one
-    //   on Helios).
+    // - fixed-base commitments (none on Helios, two on Selene);
+    // - single MSMs from host buffers, whose accumulation is pipelined with the link
+    //   (none on Helios, one on Selene).
     bool ba_set[2] = {false, false};
     uint32_t fixed_ba_rounds[2] = {0, 2};
     uint32_t host_ba_rounds[2] = {0, 1};

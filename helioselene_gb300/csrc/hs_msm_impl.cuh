@@ -10,11 +10,13 @@
 //      thread sums one segment of affine bases into an XYZZ point;
 //   3. k_merge / k_merge_heavy: buckets with several segments are folded
 //      (sequentially when few, by a block-wide tree when many);
-//   4. k_reduce_groups / k_window_chunks / k_window_sum: per window
+//   4. k_reduce_groups / k_window_chunks / k_window_sum (k_window_serial for many
+//      windows, k_window_quads instead of all for small plans): per window
 //      S = sum_j (j+1) B_j by running sums over groups of 8 buckets, then
 //      suffix scans and trees over the groups (no scalar multiples);
 //   5. k_combine: Horner over the windows, S = 2^c S + S_k (the reference's
-//      per-window doublings, :285-289) on one warp, result as canonical Jacobian.
+//      per-window doublings, :285-289) on lane-sliced elements, a cluster of blocks
+//      per MSM; result as canonical Jacobian.
 #pragma once
 
 #include <cooperative_groups.h>

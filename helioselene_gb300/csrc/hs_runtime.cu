@@ -770,8 +770,8 @@ __global__ void k_recode(const uint4 *__restrict__ scalars, uint32_t n_total, co
 // row of counts per block goes to global memory.
 //   k_digits       every scalar's signed digits, window-major, in one pass
 //   k_sort_count   count the block's keys, write its row of counts
-//   k_sort_totals  per bucket: the sum of its rows -> counts (then the scan)
-//   k_sort_offsets per bucket: each row's first slot, offsets + earlier rows
+//   k_sort_rows    per bucket: the sum of its rows -> counts (then the scan), and
+//                  after it each row's first slot, offsets + earlier rows
 //   k_sort_scatter place "index | sign" at the row's slot + running fill
 // ---------------------------------------------------------------------------
 struct SortBlock {

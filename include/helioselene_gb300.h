@@ -87,20 +87,22 @@ uint64_t hs_context_launches(const hs_context *ctx);
 void *hs_context_stream(hs_context *ctx);
 /* Bucket accumulation form of one curve's plans of at least min_entries
  * (point, window) entries: `rounds` (1..3) rounds of pairwise affine
- * additions, each round sharing one field inversion per 2048 additions
+ * additions, each round sharing one field inversion per 32768 additions
  * (Montgomery's trick, fp/include/fp_batch_invert.h:61-114, across a wave of
  * bucket additions), then an XYZZ fold of what is left; 0 keeps the XYZZ mixed
  * additions of every entry (helios/src/x64/helios_msm_vartime.cpp:296-325 is
  * the bucket loop both replace).  Results are identical either way.  Default:
- * one round on Helios and two on Selene, from 2^21 entries, except in two
- * kinds of plans where a curve's MSMs mostly run alone: fixed-base commitments
- * and single MSMs from host buffers take no round on Helios and one on
- * Selene, until this call sets the curve.  rounds = -1 restores the defaults.  Host-input calls
+ * one round on Helios and two on Selene, from 7 * 2^20 entries (2^21 for the
+ * halves of a split MSM and for a server's slots; one round for a lone MSM or a
+ * half of fewer than 2^23), except in two kinds of plans where a curve's MSMs
+ * mostly run alone: fixed-base commitments take none on Helios and two on
+ * Selene (from 2^21 entries), single MSMs from host buffers none and one,
+ * until this call sets the curve.  rounds = -1 restores the defaults.  Host-input calls
  * send their bases in two parts either way: with rounds, each part's entries
  * of a bucket form their own list, whose rounds run once that part is in. */
 int hs_context_set_batch_affine(hs_context *ctx, int curve, int rounds, size_t min_entries);
 /* set the Pippenger window width for one curve; 0 restores the built-in
- * cost model (the autotuner writes this) */
+ * widths (the autotuner writes this) */
 int hs_context_set_window(hs_context *ctx, int curve, size_t n_min, size_t n_max, int window);
 /* the same, with the batch-affine rounds (0..3) of plans whose entries lie
  * mostly in this size class (-1: the curve's setting, hs_context_set_batch_affine);
