@@ -170,7 +170,7 @@ class ClockSampler:
         try:
             self.proc = subprocess.Popen(
                 ["nvidia-smi", "-i", str(self.device), f"--query-gpu={self.FIELDS}", "--format=csv,noheader,nounits",
-                 "-lms", "50"], stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
+                 "-lms", "20"], stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
             self.thread = threading.Thread(target=self._read, daemon=True)
             self.thread.start()
         except (FileNotFoundError, OSError):
@@ -201,10 +201,10 @@ class ClockSampler:
         lines = self.lines
         note = "samples within the timed region"
         if t0 is not None:
-            inside = [ln for ts, ln in lines if t0 <= ts <= t1 + 0.05]
+            inside = [ln for ts, ln in lines if t0 <= ts <= t1 + 0.02]
             if not inside:
                 inside = [ln for ts, ln in lines if ts >= t0][:1]
-                note = "the first sample after the timed region began (region shorter than the 50 ms interval)"
+                note = "the first sample after the timed region began (region shorter than the 20 ms interval)"
             lines = inside
         else:
             lines = [ln for _, ln in lines]
