@@ -865,8 +865,8 @@ def run_scalar_mul(hs, torch, ctxs, data, n: int, flush) -> dict:
 
 
 IMAD_PER_MODSQR = {0: 88, 1: 176}  # F_p, F_q squaring: 36 products + the same reduction
-# per decoded point: x^3 - 3x + b, one 4-bit-window exponentiation (256 S + 78 M), the root check
-DECODE_SQR, DECODE_MUL = 258, 80
+# per decoded point, by curve: x^3 - 3x + b, the root by runs of ones and windows, its check
+DECODE_SQR, DECODE_MUL = (253, 255), (14, 41)
 
 
 def run_decompress(hs, torch, ctxs, data, n: int, flush, imad_peak: float) -> dict:
@@ -896,7 +896,7 @@ def run_decompress(hs, torch, ctxs, data, n: int, flush, imad_peak: float) -> di
                 ts.append(a.elapsed_time(b))
         ok = bool(torch.equal(d_out, data[curve]["d_pts"]))
         ms = min(ts)
-        work = n * (DECODE_SQR * IMAD_PER_MODSQR[curve] + DECODE_MUL * IMAD_PER_MODMUL[curve])
+        work = n * (DECODE_SQR[curve] * IMAD_PER_MODSQR[curve] + DECODE_MUL[curve] * IMAD_PER_MODMUL[curve])
         h_sc = data[curve]["h_sc"].numpy()
         h_enc = torch.empty(n * 32, dtype=torch.uint8, pin_memory=True)
         h_enc.numpy()[:] = enc
@@ -908,7 +908,7 @@ def run_decompress(hs, torch, ctxs, data, n: int, flush, imad_peak: float) -> di
         out[name] = {"points": n, "ms": ms, "points_per_s": n / (ms * 1e-3), "round_trip_exact": ok,
                      "roofline": {"bound": "imad", "achieved": work / (ms * 1e-3) / 1e12, "peak": imad_peak / 1e12,
                                   "unit": "T IMAD/s", "frac": work / (ms * 1e-3) / imad_peak if imad_peak else None,
-                                  "work": f"{DECODE_SQR} squarings + {DECODE_MUL} products per point, "
+                                  "work": f"{DECODE_SQR[curve]} squarings + {DECODE_MUL[curve]} products per point, "
                                           "IMAD-eq as for the MSM"},
                      "msm_from_encodings_e2e": {"ms": e2e * 1e3, "points_per_s": n / e2e,
                                                 "api": "hs_msm(point_fmt=HS_FMT_COMPRESSED), pinned host buffers, "
