@@ -168,3 +168,67 @@ def test_pool_window_refused_outside_range(pools):
         for bad in ((2, 12), (0, 3), (0, 17), (1, -1)):
             with pytest.raises(hs.HsError):
                 srv.set_pool_window(*bad)
+
+
+@pytest.mark.parametrize("pooled_only", [True, False])
+def test_a_burst_of_small_requests_is_batched(pools, pooled_only):
+    """a launch takes the time of several submissions, and requests go on arriving
+    meanwhile: a burst on more slots than it can fill runs at two requests a batch or more"""
+    import helioselene_gb300 as hs
+    rng = np.random.default_rng(11)
+    reqs = []
+    for i in range(200):
+        n = int(rng.integers(20, 100))
+        n_pool = n if pooled_only else n // 2
+        scal = rng.integers(0, 256, (n, 32), dtype=np.uint8)
+        reqs.append((i % 2, scal, rng.integers(0, 4096, n_pool).astype(np.uint32), pools[i % 2][:n - n_pool]))
+    want = {i: oracle.msm(c, s, np.concatenate([pools[c][idx], f]), keep_carry=True)
+            for i, (c, s, idx, f) in enumerate(reqs) if i % 20 == 7}
+    with hs.Server(0, slots=8) as srv:
+        for c in (0, 1):
+            srv.set_pool(c, pools[c])
+        batches = []
+        for _ in range(6):
+            before = srv.stats()["batches"]
+            tickets = [srv.submit(c, s, idx, f if f.size else None) for c, s, idx, f in reqs]
+            got = [srv.wait(t)[0] for t in tickets]
+            batches.append(srv.stats()["batches"] - before)
+            assert all(got[i] == w for i, w in want.items())
+    assert min(batches) <= len(reqs) // 2, batches
+
+
+def test_pools_and_rules_while_batches_are_launched(pools):
+    """window rules may change at any time and pools only while idle, also while the
+    scheduler is launching; every result is the same"""
+    import threading
+
+    import helioselene_gb300 as hs
+    rng = np.random.default_rng(12)
+    reqs = make_requests(rng, pools, 40, 4096)
+    with hs.Server(0, slots=4) as srv:
+        for c in (0, 1):
+            srv.set_pool(c, pools[c])
+        stop, changes = threading.Event(), [0]
+
+        def change():
+            while not stop.is_set():
+                srv.set_window(changes[0] % 2, 1, 1 << 20, 5 + changes[0] % 9)
+                srv.set_window(changes[0] % 2, 0, 0, 0)
+                changes[0] += 1
+
+        t = threading.Thread(target=change)
+        t.start()
+        try:
+            for _ in range(5):
+                tickets = [srv.submit(r["curve"], r["scalars"], r["idx"], r["fresh"]) for r in reqs]
+                try:
+                    srv.set_pool(0, pools[0])  # refused unless everything is done already
+                except hs.HsError:
+                    pass
+                got = [srv.wait(k)[0] for k in tickets]
+                assert [i for i, (g, r) in enumerate(zip(got, reqs)) if g != r["want"]] == []
+        finally:
+            stop.set()
+            t.join()
+        assert changes[0] > 0
+        srv.set_pool(0, pools[0])
