@@ -9,7 +9,11 @@
 // product, so an addition takes about 1.2 / 1.6 us against 3.5 / 5.3 us on one
 // thread.  Every function is called by all 32 lanes of a warp (eight quads),
 // branches on warp votes only, and is complete: identity operands and equal or
-// opposite points are handled.  The two operations are out of line, the points
+// opposite points are handled, and where no quad of the warp has two points to add
+// (or one to double) nothing is computed: small scalars leave most buckets empty, and
+// one F_p MSM of 65536 points with scalars 0 and 1 took 346 us, 96 of them in level 2
+// on identities (305 with one thread per point, which leaves early), and 271 so.
+// The two operations are out of line, the points
 // passed by value in registers: a kernel's many uses then share one body, which
 // stays in the instruction cache.  Level 2 of one MSM of 2^20 points (F_p / F_q):
 // 184 / 287 us with one thread per point, 160 / 217 with inlined quads, 139 / 177
@@ -73,6 +77,8 @@ struct Quad {
     {
         // lane 0: T = (X - ZZ)(X + ZZ); lane 1: V = (2Y)^2
         const Fe o = bcast(p, 2);
+        if (__all_sync(ALL, F::is_exact_zero(o)))
+            return p;  // eight identities
         const Fe u = F::dbl(p);
         const Fe r1 = F::mul(sel(j == 0, F::sub(p, o), u), sel(j == 0, F::add(p, o), u));
         const Fe v = bcast(r1, 1), t = bcast(r1, 0);
@@ -105,6 +111,9 @@ struct Quad {
         // (flags are shuffles: taken on every lane, never behind a short-circuit)
         const bool p_inf = is_inf(p), q_zero = is_inf(q);
         const bool q_inf = !take || (!MIXED && q_zero);
+        const Fe qv = MIXED ? sel(j < 2, q, F::one()) : q;
+        if (__all_sync(ALL, p_inf || q_inf))  // no quad has two points to add
+            return q_inf ? p : qv;
         // U1 = X1 ZZ2, S1 = Y1 ZZZ2, U2 = X2 ZZ1, S2 = Y2 ZZZ1 on lanes 0..3 (MIXED: U1 = X1, S1 = Y1)
         Fe r1 = F::mul(p, shx(q, 2));
         if (MIXED)
@@ -136,7 +145,6 @@ struct Quad {
             const Fe two = dbl_v(z, j);
             r = same_x ? sel(same_y, two, F::zero()) : r;
         }
-        const Fe qv = MIXED ? sel(j < 2, q, F::one()) : q;
         return q_inf ? p : sel(p_inf, qv, r);
     }
 };
