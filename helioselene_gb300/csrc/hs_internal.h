@@ -215,6 +215,14 @@ struct BatchPlan {
     // part-1 segment continues the sum of its first part-0 segment.
     uint32_t part_slice = 0;
     uint64_t entries_bound = 0; // sum n_i * W_i
+    uint64_t buckets = 0;       // sum W_i * B_i: NB where it fits
+    // Entries and buckets are indexed with 31 bits, the sort's rows of counts with 32; a
+    // plan beyond that is not launched (NB and the offsets below it may have wrapped).
+    bool fits() const
+    {
+        return entries_bound < 0x80000000ull && buckets < 0x80000000ull &&
+               (!smem_sort() || cnt_len <= 0xffffffffull);
+    }
     // the algorithmic count of (point, window) entries: n_i * ceil(256/c_i) per
     // MSM (the full windows of a 256-bit scalar, not the carry window), the
     // unit of the pinned work figure that instrumentation reports
@@ -290,6 +298,8 @@ BatchPlan make_batch_plan(const Context &ctx, int curve, const size_t *sizes, ui
                           bool decoded = false);
 // count fixed-base MSMs of n table generators each (window c), scalars back to back
 BatchPlan make_fixed_plan(int curve, size_t n, int c, uint32_t count);
+// commitments of one launch sequence of such a plan, of count in all
+size_t fixed_chunk(size_t n, int c, size_t count);
 // M MSMs over rows of one window-multiple table (window c) named by index lists
 // (fixed = 2): sizes[i] generators each, scalars and indices back to back
 BatchPlan make_indexed_plan(const Context &ctx, int curve, const size_t *sizes, uint32_t M, int c);

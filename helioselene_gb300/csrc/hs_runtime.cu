@@ -361,6 +361,7 @@ BatchPlan make_batch_plan(const Context &ctx, int curve, const size_t *sizes, ui
         p.entries_pinned += (uint64_t)n * (uint64_t)((256 + c - 1) / c);
     }
     p.n_total = (uint32_t)pt;
+    p.buckets = nb;
     p.NB = (uint32_t)nb;
     p.G = (uint32_t)g;
     p.WS = (uint32_t)ws;
@@ -428,6 +429,7 @@ BatchPlan make_fixed_plan(int curve, size_t n, int c, uint32_t count)
     const uint64_t ent = (uint64_t)count * n * W;
     p.entries_pinned = (uint64_t)count * n * (uint64_t)((256 + c - 1) / c);
     p.n_total = (uint32_t)(count * n);
+    p.buckets = (uint64_t)count * B;
     p.NB = count * B;
     p.G = count * (B / m0);
     p.WS = count;
@@ -439,6 +441,13 @@ BatchPlan make_fixed_plan(int curve, size_t n, int c, uint32_t count)
     plan_chunks(p);
     plan_sort(p);
     return p;
+}
+
+size_t fixed_chunk(size_t n, int c, size_t count)
+{
+    const uint64_t per = (uint64_t)n * (uint64_t)((257 + c - 1) / c);
+    const uint64_t by_entries = (1ull << 29) / std::max<uint64_t>(1, per), by_buckets = 0x7fffffffull >> (c - 1);
+    return (size_t)std::max<uint64_t>(1, std::min<uint64_t>(count, std::min(by_entries, by_buckets)));
 }
 
 BatchPlan make_indexed_plan(const Context &ctx, int curve, const size_t *sizes, uint32_t M, int c)
@@ -476,6 +485,7 @@ BatchPlan make_indexed_plan(const Context &ctx, int curve, const size_t *sizes, 
     const uint64_t ent = pt * W;
     p.entries_pinned = pt * (uint64_t)((256 + c - 1) / c);
     p.n_total = (uint32_t)pt;
+    p.buckets = (uint64_t)M * B;
     p.NB = M * B;
     p.G = M * (B / m0);
     p.WS = M;
@@ -523,6 +533,7 @@ BatchPlan make_window_plan(int curve, size_t n, int c, uint32_t w_lo, uint32_t w
         p.entries_pinned = hi > w_lo ? (uint64_t)n * (hi - w_lo) : 0;
     }
     p.n_total = (uint32_t)n;
+    p.buckets = (uint64_t)w_cnt * d.B;
     p.NB = w_cnt * d.B;
     p.G = w_cnt * d.T;
     p.WS = w_cnt;
@@ -2917,7 +2928,7 @@ int hs_msm_batch_device(hs_context *h, int curve, const size_t *sizes, size_t co
     std::lock_guard<std::mutex> lk(ctx.mu);
     DeviceGuard g(ctx.device);
     const BatchPlan p = make_batch_plan(ctx, curve, sizes, (uint32_t)count);
-    if ((uint64_t)p.NB >= 0x80000000ull || p.entries_bound >= 0x80000000ull)
+    if (!p.fits())
         return fail_msg(ctx, HS_ERANGE, "batch too large for one launch sequence");
     BatchBuffers b;
     int rc = reserve_batch(ctx, p, 0, b, nullptr);
@@ -2961,7 +2972,7 @@ int hs_msm_batch(hs_context *h, const hs_msm_desc *descs, size_t count, int poin
         if (idx[k].empty())
             continue;
         plans[k] = make_batch_plan(ctx, k, sizes[k].data(), (uint32_t)idx[k].size());
-        if (plans[k].entries_bound >= 0x80000000ull)
+        if (!plans[k].fits())
             return fail_msg(ctx, HS_ERANGE, "batch too large for one launch sequence");
         const size_t t = std::max<size_t>(1, totals[k]);
         stage[k] = align256(t * 32) + align256(t * 64) + (point_fmt == HS_FMT_AFFINE ? 0 : align256(t * pb)) +
@@ -3345,8 +3356,7 @@ static BatchPlan fixed_plan(const Context &ctx, const hs_fixed_base *fb, uint32_
 static int fixed_commit_chunks(Context &ctx, const hs_fixed_base *fb, const uint8_t *d_scalars, size_t count,
                                uint8_t *d_out, int out_fmt)
 {
-    const uint64_t per = (uint64_t)fb->n_gen * fb->W;
-    const size_t chunk = (size_t)std::max<uint64_t>(1, std::min<uint64_t>(count, (1ull << 29) / per));
+    const size_t chunk = fixed_chunk(fb->n_gen, fb->c, count);
     const BatchPlan big = fixed_plan(ctx, fb, (uint32_t)chunk);
     const bool aff = out_fmt == HS_FMT_AFFINE;
     // affine results: Jacobian first, then one shared inversion per 16 commitments
@@ -3409,8 +3419,7 @@ int hs_fixed_base_commit(hs_context *h, const hs_fixed_base *fb, const uint8_t *
     std::lock_guard<std::mutex> lk(ctx.mu);
     DeviceGuard g(ctx.device);
     const CurveOps &ops = curve_ops(fb->curve);
-    const uint64_t per = (uint64_t)fb->n_gen * fb->W;
-    const size_t chunk = (size_t)std::max<uint64_t>(1, std::min<uint64_t>(count, (1ull << 29) / per));
+    const size_t chunk = fixed_chunk(fb->n_gen, fb->c, count);
     const size_t ob = fmt_bytes(out_fmt);
     // staging for one chunk: scalars in the device layout, Jacobian results, formatted results
     const size_t sc_bytes = align256(chunk * fb->n_gen * 32);

@@ -54,7 +54,7 @@ __global__ void k_gather_pool(const uint4 *__restrict__ pool, const uint32_t *__
 
 using Clock = std::chrono::steady_clock;
 
-// one launch sequence indexes its (point, window) entries with 31 bits
+// one launch sequence indexes its (point, window) entries and its buckets with 31 bits
 constexpr uint64_t BATCH_ENTRIES_MAX = 0x7fffffffull;
 
 struct ReqState {
@@ -62,6 +62,7 @@ struct ReqState {
     size_t n = 0;
     bool table = false;    // pooled bases only, computed over the pool's window table
     uint64_t entries = 0;  // n x windows under the slots' window rules at submission
+    uint64_t buckets = 0;  // of those windows, or of the pool table's one
     Clock::time_point submitted;
     double latency_ms = 0.0;
     int status = 1;  // 1 = pending, else HS_OK / error
@@ -129,16 +130,22 @@ static bool table_form(const Server &S, const hs_request &q)
     return S.pools[q.curve].table && q.n_pool && !q.n_fresh;
 }
 
-// (point, window) entries of a request under the slots' window rules, or the
-// pool table's windows: what a batch of requests is bounded by (a plan whose own
-// widths exceed the bound takes these)
-static uint64_t request_entries(const Server &S, const hs_request &q)
+// (point, window) entries and buckets of a request under the slots' window rules, or
+// the pool table's windows: what a batch of requests is bounded by (a plan whose own
+// widths exceed the bound of the entries takes these; the buckets are the most of any)
+static void request_size(const Server &S, ReqState &r)
 {
-    const size_t n = q.n_pool + q.n_fresh;
-    if (table_form(S, q))
-        return (uint64_t)n * S.pools[q.curve].W;
-    const int c = choose_window(S.slots[0]->ctx, q.curve, n ? n : 1, Widths::fewest_ops);
-    return (uint64_t)n * (uint64_t)((257 + c - 1) / c);
+    if (r.table) {
+        r.entries = (uint64_t)r.n * S.pools[r.req.curve].W;
+        r.buckets = 1ull << (S.pools[r.req.curve].c - 1);
+        return;
+    }
+    const int c = choose_window(S.slots[0]->ctx, r.req.curve, r.n ? r.n : 1, Widths::fewest_ops);
+    r.entries = (uint64_t)r.n * (uint64_t)((257 + c - 1) / c);
+    for (Widths use : {Widths::alone, Widths::few, Widths::many, Widths::fewest_ops}) {
+        const int w = choose_window(S.slots[0]->ctx, r.req.curve, r.n ? r.n : 1, use);
+        r.buckets = std::max(r.buckets, (uint64_t)((257 + w - 1) / w) << (w - 1));
+    }
 }
 
 static size_t batch_stage_bytes(size_t total, size_t total_pool, size_t msms, size_t ob)
@@ -221,7 +228,7 @@ static Launch launch_table(const Server &S, Slot &s, const std::vector<const Req
     }
     Context &ctx = s.ctx;
     const BatchPlan p = make_indexed_plan(ctx, curve, sizes.data(), M, pool.c);
-    if (p.entries_bound > BATCH_ENTRIES_MAX)
+    if (!p.fits())
         return Launch{false, HS_ERANGE, 0};
     // staging: scalars, indices, M results
     const size_t extra = align256(std::max<size_t>(1, tp) * 32) + align256(std::max<size_t>(1, tp) * 4) +
@@ -291,7 +298,7 @@ static Launch launch(const Server &S, Slot &s, const std::vector<const ReqState 
     }
     Context &ctx = s.ctx;
     const BatchPlan p = make_batch_plan(ctx, curve, sizes.data(), (uint32_t)sizes.size());
-    if (p.entries_bound > BATCH_ENTRIES_MAX)  // window rules changed since submission
+    if (!p.fits())  // window rules changed since submission
         return Launch{false, HS_ERANGE, 0};
     const size_t extra = batch_stage_bytes(total, total_pool, batch.size(), ob);
     const size_t bytes = batch_bytes(p) + extra + 2048;
@@ -441,18 +448,20 @@ static void scheduler(Server *Sp)
             std::vector<uint64_t> batch;
             std::vector<const ReqState *> reqs;  // (a map's elements stay where they are while others are added)
             size_t pts = 0;
-            uint64_t ent = 0;
+            uint64_t ent = 0, buckets = 0;
             std::deque<uint64_t> rest;
             while (!S.queue.empty()) {
                 const uint64_t t = S.queue.front();
                 S.queue.pop_front();
                 const ReqState &r = S.reqs.at(t);
                 if (r.req.curve == curve && r.table == form && batch.size() < S.cfg.max_batch_msms &&
-                    (batch.empty() || (pts + r.n <= S.cfg.max_batch_points && ent + r.entries <= BATCH_ENTRIES_MAX))) {
+                    (batch.empty() || (pts + r.n <= S.cfg.max_batch_points && ent + r.entries <= BATCH_ENTRIES_MAX &&
+                                       buckets + r.buckets <= BATCH_ENTRIES_MAX))) {
                     batch.push_back(t);
                     reqs.push_back(&r);
                     pts += r.n;
                     ent += r.entries;
+                    buckets += r.buckets;
                 } else {
                     rest.push_back(t);
                 }
@@ -696,16 +705,16 @@ int hs_server_submit(hs_server *h, const hs_request *req, uint64_t *ticket)
         if (S.pools[req->curve].gen == gen)
             break;
     }
-    const uint64_t entries = request_entries(S, *req);
-    if (entries > BATCH_ENTRIES_MAX)
-        return HS_ERANGE;
-    const uint64_t t = S.next_ticket++;
-    ReqState &r = S.reqs[t];
+    ReqState r;
     r.req = *req;
     r.n = n;
     r.table = table_form(S, *req);
-    r.entries = entries;
+    request_size(S, r);
+    if (r.entries > BATCH_ENTRIES_MAX)
+        return HS_ERANGE;
     r.submitted = Clock::now();
+    const uint64_t t = S.next_ticket++;
+    S.reqs[t] = r;
     S.queue.push_back(t);
     S.stats.submitted++;
     *ticket = t;

@@ -94,3 +94,14 @@ def test_per_size_window_rules_in_one_batch(ctx):
         assert ctx.msm_batch(items, HS_AFF, HS_COMPRESSED) == want
     finally:
         ctx.set_window(1, 0, 0, 0)
+
+
+def test_batch_beyond_one_launch_sequence_is_refused(ctx):
+    """5.2 million MSMs of one point: fewer entries than 2^31, but more buckets than 2^32"""
+    import torch
+
+    import helioselene_gb300 as hs
+    buf = torch.zeros(256, dtype=torch.uint8, device="cuda:0")
+    with pytest.raises(hs.HsError) as e:
+        ctx.msm_batch_device(0, [1] * 5_200_000, buf.data_ptr(), buf.data_ptr(), buf.data_ptr(), hs.FMT_COMPRESSED)
+    assert e.value.status == -6
