@@ -295,11 +295,17 @@ static uint32_t seg_cap(uint64_t ent, uint64_t nb)
 // second round pays for one MSM in long lists of many entries (Selene on GB300, us:
 // 2^21 points 4657 with one round, 4525 with two; 2^19 1762 and 1853; 2^18 1280 and
 // 1455); the MSMs of a batch, mostly beside the other curve's, keep theirs.
+// A bucket's list is padded to a multiple of 2 or 4, so sparse lists are mostly padding:
+// 4096 x 64 points in 32 buckets a window (2 entries each) 6835 us without, 7767 with
+// two; in 16 buckets (4 each) 6623 and 6992; 8192 x 200 in 32 (6 each) 19549 and 19321.
+// And the workspace of many tiny MSMs would be mostly that of the rounds: 281073 of at
+// most 5 points 92 GB with two, 19 without.
 constexpr uint64_t BA_TWO_MIN_ENTRIES = uint64_t(1) << 23;
+constexpr uint64_t BA_MIN_PER_BUCKET = 5;
 
 static uint32_t default_rounds(const BatchPlan &p, uint32_t rounds, uint64_t least)
 {
-    if (p.entries_bound < least)
+    if (p.entries_bound < least || p.entries_bound < BA_MIN_PER_BUCKET * p.buckets)
         return 0;
     return p.M > 1 || p.entries_bound >= BA_TWO_MIN_ENTRIES ? rounds : std::min<uint32_t>(rounds, 1);
 }

@@ -83,3 +83,13 @@ def test_fixed_base_chunks(plan, n, window, count, chunk):
     got, fits = plan("fixed", n, window, count).split()
     assert (int(got), int(fits)) == (chunk, 1)
 
+
+
+# curve 1 takes two rounds by default; sparse lists (at most 4 entries a bucket) none, and
+# without them an MSM of three points takes less than the 128 KB that 33 windows of 128
+# buckets take
+@pytest.mark.parametrize("count,n,rounds", [(8192, 200, 2), (4096, 64, 0), (281073, 3, 0), (800000, 3, 0)])
+def test_rounds_and_workspace_of_many_small_msms(plan, count, n, rounds):
+    fits, _, _, got, bytes_, _ = plan("batch", 1, 0, count, n).split()
+    assert (int(fits), int(got)) == (1, rounds)
+    assert n > 3 or int(bytes_) < count * 128000, bytes_
