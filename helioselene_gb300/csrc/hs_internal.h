@@ -300,6 +300,10 @@ BatchPlan make_batch_plan(const Context &ctx, int curve, const size_t *sizes, ui
 BatchPlan make_fixed_plan(int curve, size_t n, int c, uint32_t count);
 // commitments of one launch sequence of such a plan, of count in all
 size_t fixed_chunk(size_t n, int c, size_t count);
+// such a plan with the context's bucket accumulation form, and the workspace that count
+// commitments in chunks need
+BatchPlan fixed_plan(const Context &ctx, int curve, size_t n, int c, uint32_t count);
+size_t fixed_workspace(const Context &ctx, int curve, size_t n, int c, size_t count);
 // M MSMs over rows of one window-multiple table (window c) named by index lists
 // (fixed = 2): sizes[i] generators each, scalars and indices back to back
 BatchPlan make_indexed_plan(const Context &ctx, int curve, const size_t *sizes, uint32_t M, int c);

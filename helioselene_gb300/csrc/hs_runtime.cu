@@ -456,6 +456,14 @@ size_t fixed_chunk(size_t n, int c, size_t count)
     return (size_t)std::max<uint64_t>(1, std::min<uint64_t>(count, std::min(by_entries, by_buckets)));
 }
 
+BatchPlan fixed_plan(const Context &ctx, int curve, size_t n, int c, uint32_t count)
+{
+    BatchPlan p = make_fixed_plan(curve, n, c, count);
+    const int k = curve == HS_SELENE ? 1 : 0;
+    plan_batch_affine(p, ctx.ba_set[k] ? ctx.ba_rounds[k] : ctx.fixed_ba_rounds[k], ctx.ba_min_entries[k]);
+    return p;
+}
+
 BatchPlan make_indexed_plan(const Context &ctx, int curve, const size_t *sizes, uint32_t M, int c)
 {
     BatchPlan p;
@@ -616,6 +624,14 @@ size_t batch_bytes(const BatchPlan &p)
         b += 8 * 256;
     }
     return b + 16 * 256;
+}
+
+// (the last, smaller chunk may have smaller groups and so more of them than the others)
+size_t fixed_workspace(const Context &ctx, int curve, size_t n, int c, size_t count)
+{
+    const size_t chunk = fixed_chunk(n, c, count), rest = count % chunk;
+    const size_t b = batch_bytes(fixed_plan(ctx, curve, n, c, (uint32_t)chunk));
+    return rest ? std::max(b, batch_bytes(fixed_plan(ctx, curve, n, c, (uint32_t)rest))) : b;
 }
 
 bool carve(DeviceArena &a, const BatchPlan &p, BatchBuffers &b)
@@ -3348,32 +3364,23 @@ int hs_fixed_base_create(hs_context *h, int curve, const void *generators, int p
     return HS_OK;
 }
 
-// a chunk of `count` commitments, with the curve's bucket accumulation form
-static BatchPlan fixed_plan(const Context &ctx, const hs_fixed_base *fb, uint32_t count)
-{
-    BatchPlan p = make_fixed_plan(fb->curve, fb->n_gen, fb->c, count);
-    const int k = fb->curve == HS_SELENE ? 1 : 0;
-    plan_batch_affine(p, ctx.ba_set[k] ? ctx.ba_rounds[k] : ctx.fixed_ba_rounds[k], ctx.ba_min_entries[k]);
-    return p;
-}
-
 // Run count fixed-base commitments whose scalars are at d_scalars (count x n_gen
 // x 32 bytes on the device) in chunks bounded by the entry count; results to d_out.
 static int fixed_commit_chunks(Context &ctx, const hs_fixed_base *fb, const uint8_t *d_scalars, size_t count,
                                uint8_t *d_out, int out_fmt)
 {
     const size_t chunk = fixed_chunk(fb->n_gen, fb->c, count);
-    const BatchPlan big = fixed_plan(ctx, fb, (uint32_t)chunk);
     const bool aff = out_fmt == HS_FMT_AFFINE;
     // affine results: Jacobian first, then one shared inversion per 16 commitments
     const size_t extra = aff ? align256(count * 120) + align256(count * 32) : 0;
-    HS_CU(ctx.arena.reserve(batch_bytes(big) + extra + 2048), "workspace allocation");
+    HS_CU(ctx.arena.reserve(fixed_workspace(ctx, fb->curve, fb->n_gen, fb->c, count) + extra + 2048),
+          "workspace allocation");
     const size_t ob = aff ? 120 : fmt_bytes(out_fmt);
     uint8_t *d_jac = nullptr;
     void *d_scr = nullptr;
     for (size_t j0 = 0; j0 < count; j0 += chunk) {
         const size_t cnt = std::min(chunk, count - j0);
-        const BatchPlan p = fixed_plan(ctx, fb, (uint32_t)cnt);
+        const BatchPlan p = fixed_plan(ctx, fb->curve, fb->n_gen, fb->c, (uint32_t)cnt);
         ctx.arena.reset();
         if (aff) {  // results and scratch live at the front of the arena, below the batch workspace
             d_jac = (uint8_t *)ctx.arena.take(count * 120);
@@ -3430,12 +3437,12 @@ int hs_fixed_base_commit(hs_context *h, const hs_fixed_base *fb, const uint8_t *
     // staging for one chunk: scalars in the device layout, Jacobian results, formatted results
     const size_t sc_bytes = align256(chunk * fb->n_gen * 32);
     const size_t extra = sc_bytes + align256(chunk * 120) + align256(chunk * ob) + align256(chunk * 32) + 256;
+    const size_t work = fixed_workspace(ctx, fb->curve, fb->n_gen, fb->c, count);
     std::vector<uint8_t> host(count * ob);
     for (size_t j0 = 0; j0 < count; j0 += chunk) {
         const size_t cnt = std::min(chunk, count - j0);
-        const BatchPlan big = fixed_plan(ctx, fb, (uint32_t)chunk);
-        HS_CU(ctx.arena.reserve(batch_bytes(big) + align256(extra) + 1024), "workspace allocation");
-        const BatchPlan p = fixed_plan(ctx, fb, (uint32_t)cnt);
+        HS_CU(ctx.arena.reserve(work + align256(extra) + 1024), "workspace allocation");
+        const BatchPlan p = fixed_plan(ctx, fb->curve, fb->n_gen, fb->c, (uint32_t)cnt);
         BatchBuffers b;
         if (!carve(ctx.arena, p, b))
             return fail_msg(ctx, HS_ENOMEM, "workspace carve");

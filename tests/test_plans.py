@@ -10,6 +10,7 @@ from conftest import ROOT
 from test_pull_pieces import cuda_include
 
 PROGRAM = r"""
+#include <algorithm>
 #include <cstdio>
 #include <string>
 #include "hs_internal.h"
@@ -38,6 +39,18 @@ int main(int argc, char **argv)
         const size_t chunk = fixed_chunk(arg(2), (int)arg(3), arg(4));
         const BatchPlan p = make_fixed_plan(0, arg(2), (int)arg(3), (uint32_t)chunk);
         std::printf("%zu %d\n", chunk, (int)p.fits());
+    } else if (what == "chunks") {  // generators, window, count, rounds
+        ctx.ba_set[0] = true;
+        ctx.ba_rounds[0] = (uint32_t)arg(5);
+        const size_t n = arg(2), count = arg(4), chunk = fixed_chunk(n, (int)arg(3), count);
+        for (size_t j = 0; j < count; j += chunk) {
+            DeviceArena a;  // nothing is read or written: the buffers are only laid out
+            a.base = reinterpret_cast<char *>(256);
+            a.cap = fixed_workspace(ctx, 0, n, (int)arg(3), count) + 1024;
+            BatchBuffers b;
+            std::printf("%d", (int)carve(a, fixed_plan(ctx, 0, n, (int)arg(3), (uint32_t)std::min(chunk, count - j)), b));
+            a.base = nullptr;
+        }
     }
     return 0;
 }
@@ -93,3 +106,12 @@ def test_rounds_and_workspace_of_many_small_msms(plan, count, n, rounds):
     fits, _, _, got, bytes_, _ = plan("batch", 1, 0, count, n).split()
     assert (int(fits), int(got)) == (1, rounds)
     assert n > 3 or int(bytes_) < count * 128000, bytes_
+
+
+# chunks of 1024 commitments whose last one has groups half the size
+@pytest.mark.parametrize("rounds", [0, 1, 2])
+@pytest.mark.parametrize("n,window,count", [(26214, 13, 1024 + 1023), (26214, 13, 2048), (5000, 10, 4129 + 4095),
+                                            (228, 9, 200000)])
+def test_every_chunk_of_commitments_has_its_workspace(plan, n, window, count, rounds):
+    out = plan("chunks", n, window, count, rounds)
+    assert len(out) >= 2 and set(out) == {"1"}, out
