@@ -41,10 +41,6 @@ struct SeleneCurve {
     static constexpr int SSWU_Z = -4;  // selene/src/x64/selene_map_to_curve.cpp
 };
 
-struct Affine {
-    Fe x, y;
-};
-
 struct Xyzz {
     Fe X, Y, ZZ, ZZZ;
 };
@@ -200,14 +196,6 @@ struct Group {
         return 0;
     }
 
-    __device__ __forceinline__ static Xyzz neg(const Xyzz &p)
-    {
-        Xyzz r = p;
-        if (!is_inf(p))
-            r.Y = F::neg(p.Y);
-        return r;
-    }
-
     // ---- Jacobian points (x = X/Z^2, y = Y/Z^3; the identity is Z exactly zero), for
     // chains of doublings: dbl-2001-b is 3M + 5S against XYZZ's 7M + 2S ----
     struct Jac {
@@ -274,21 +262,6 @@ struct Group {
         Z = F::mul(p.ZZ, p.ZZZ);
         X = F::mul(F::mul(p.X, p.ZZ), zzz2);
         Y = F::mul(F::mul(p.Y, F::mul(zz2, p.ZZ)), zzz2);
-    }
-
-    // XYZZ -> canonical affine (one inversion); identity -> (0,0)
-    __device__ static Affine to_affine(const Xyzz &p)
-    {
-        Affine a;
-        if (is_inf(p)) {
-            a.x = F::zero();
-            a.y = F::zero();
-            return a;
-        }
-        Fe inv = F::inv(F::mul(p.ZZ, p.ZZZ));
-        a.x = F::canon(F::mul(F::mul(p.X, p.ZZZ), inv));
-        a.y = F::canon(F::mul(F::mul(p.Y, p.ZZ), inv));
-        return a;
     }
 };
 
