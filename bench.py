@@ -46,7 +46,11 @@ METRIC = "MSM points/sec at n=2^20 (both curves, bit-exact); batched-serving MSM
 WORKLOAD = ("Helios + Selene vartime Pippenger MSM, n=2^20 each; scalars uniform mod order; "
             "SWU-derived affine bases; 1% edge slices (zero, order-1, repeated base, top-window-only)")
 from helioselene_gb300.workload import BENCH_SEED as SEED  # noqa: E402
-IMAD_PER_MODMUL = {0: 144, 1: 232}  # F_p, F_q: 2 IMAD per 32x32->64 product
+# the pinned work unit of one field product (F_p, F_q): 2 IMAD per 32x32->64 product
+IMAD_PER_MODMUL = {0: 144, 1: 232}
+# what the kernels execute: 64 products and a fold of 8 (F_p) or 32 (F_q), a square 36
+# instead of 64; a difference of two products shares one fold on F_q
+EXEC_MUL, EXEC_SQR, EXEC_MUL_SUB = {0: 144, 1: 192}, {0: 88, 1: 136}, {0: 288, 1: 320}
 # dram__bytes_read.sum + dram__bytes_write.sum of the bucket-accumulation phase of
 # one MSM at n = 2^20 (Helios, Selene), from ncu --set full captures of this
 # workload, by accumulation form (batch-affine rounds): 0 is k_accumulate, 1 is
@@ -867,7 +871,6 @@ def run_scalar_mul(hs, torch, ctxs, data, n: int, flush) -> dict:
     return out
 
 
-IMAD_PER_MODSQR = {0: 88, 1: 176}  # F_p, F_q squaring: 36 products + the same reduction
 # per decoded point, by curve: x^3 - 3x + b, the root by runs of ones and windows, its check
 DECODE_SQR, DECODE_MUL = (253, 255), (14, 41)
 
@@ -899,7 +902,7 @@ def run_decompress(hs, torch, ctxs, data, n: int, flush, imad_peak: float) -> di
                 ts.append(a.elapsed_time(b))
         ok = bool(torch.equal(d_out, data[curve]["d_pts"]))
         ms = min(ts)
-        work = n * (DECODE_SQR[curve] * IMAD_PER_MODSQR[curve] + DECODE_MUL[curve] * IMAD_PER_MODMUL[curve])
+        work = n * (DECODE_SQR[curve] * EXEC_SQR[curve] + DECODE_MUL[curve] * EXEC_MUL[curve])
         h_sc = data[curve]["h_sc"].numpy()
         h_enc = torch.empty(n * 32, dtype=torch.uint8, pin_memory=True)
         h_enc.numpy()[:] = enc
@@ -912,7 +915,7 @@ def run_decompress(hs, torch, ctxs, data, n: int, flush, imad_peak: float) -> di
                      "roofline": {"bound": "imad", "achieved": work / (ms * 1e-3) / 1e12, "peak": imad_peak / 1e12,
                                   "unit": "T IMAD/s", "frac": work / (ms * 1e-3) / imad_peak if imad_peak else None,
                                   "work": f"{DECODE_SQR[curve]} squarings + {DECODE_MUL[curve]} products per point, "
-                                          "IMAD-eq as for the MSM"},
+                                          "IMAD-eq as executed"},
                      "msm_from_encodings_e2e": {"ms": e2e * 1e3, "points_per_s": n / e2e,
                                                 "api": "hs_msm(point_fmt=HS_FMT_COMPRESSED), pinned host buffers, "
                                                        "32 B scalar + 32 B encoding per point"}}
@@ -922,9 +925,9 @@ def run_decompress(hs, torch, ctxs, data, n: int, flush, imad_peak: float) -> di
 def executed_per_entry(rounds: int, curve: int) -> float:
     """IMAD-equivalents executed per (point, window) entry by the accumulation with
     `rounds` batch-affine rounds: round r adds 2^-r pairs per entry at 5M + 1S, the
-    fold 2^-rounds items per entry at 8M + 2S"""
-    m, s = IMAD_PER_MODMUL[curve], IMAD_PER_MODSQR[curve]
-    pair, madd = 5 * m + s, 8 * m + 2 * s
+    fold 2^-rounds items per entry at 6M + 2S and a difference of two products"""
+    m, s = EXEC_MUL[curve], EXEC_SQR[curve]
+    pair, madd = 5 * m + s, 6 * m + 2 * s + EXEC_MUL_SUB[curve]
     return sum(pair / 2**r for r in range(1, rounds + 1)) + madd / 2**rounds
 
 
@@ -954,7 +957,8 @@ def probe_rates(rates: dict, torch, local: int, clk: dict) -> dict:
     mhz = clk.get("sm_mhz") or clk.get("sm_max_mhz")
     out = {"sm_count": sms, "sm_mhz": mhz, "unit": "instructions per SM per clock",
            "note": "mad_lo_hi: alternating mad.lo/mad.hi (1 IMAD-eq each); mad_wide: mad.wide.u32 (one 32x32->64 "
-                   "product, 2 IMAD-eq); peak = max(mad_lo_hi, 2 x mad_wide) x SMs x clock"}
+                   "product, 2 IMAD-eq); mad_hi: as long on the pipe as a product; peak = max(mad_lo_hi, 2 x mad_wide, "
+                   "2 x mad_hi) x SMs x clock"}
     for k, v in rates.items():
         out[k] = round(v / (sms * mhz * 1e6), 2) if mhz else None
     return out
@@ -1304,13 +1308,15 @@ def run_ours(args) -> None:
                          "ba_rounds": {"helios": rr[0], "selene": rr[1]},
                          "work": "point-window entries x 6 modmul (batch-affine bucket add) x IMAD-eq per modmul "
                                  "(F_p 144, F_q 232), summed over one Helios and one Selene launch",
-                         "peak_source": "measured in this run by hs_measure_imad_peak (the faster of mad.lo/mad.hi "
-                                        "and mad.wide.u32 chains on every SM)",
+                         "peak_source": "measured in this run by hs_measure_imad_peak (the fastest of mad.lo/mad.hi, "
+                                        "mad.wide.u32 and mad.hi chains on every SM)",
                          "accumulate_ms_per_launch": acc_ms,
                          "executed_frac": (prof_total["executed"] / (prof_total["ms"] * 1e-3) / imad_peak
                                            if imad_peak and prof_total["ms"] > 0 else None),
-                         "executed_note": "the same launches counted with the products they execute: XYZZ mixed "
-                                          "addition 8 products + 2 squares per item; a batch-affine pair 5 "
+                         "executed_note": "the same launches counted with the products they execute (F_p 144, F_q "
+                                          "192 IMAD-eq; squares 88, 136): XYZZ mixed "
+                                          "addition 8 products (two of them under one fold on F_q) + 2 squares "
+                                          "per item; a batch-affine pair 5 "
                                           "products + 1 square (prefix, walk back, lambda, y) plus the shared "
                                           "inversion",
                          "whole_msm_frac": whole / imad_peak if imad_peak else None,

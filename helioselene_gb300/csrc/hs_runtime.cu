@@ -1596,8 +1596,11 @@ void prof_end(Context &ctx, cudaEvent_t ev0, uint64_t entries)
 // Probes of the integer-multiply pipe, 8 independent chains per thread:
 // MODE 0 alternates mad.lo / mad.hi (one 32x32->64 product = 2 IMAD-equivalents
 // per pair), MODE 1 is mad.lo alone, MODE 2 mad.hi alone; k_imad_wide_peak runs
-// mad.wide.u32 chains (the whole product in one instruction).  The ceiling is
-// the faster of the two product forms.
+// mad.wide.u32 chains (the whole product in one instruction).  mad.hi and mad.wide
+// hold the pipe for the same time, and the assembler turns part of a probe's
+// mad.wide into a product and adds, so the rate of mad.hi is the ceiling of products:
+// 31.2 per clock and SM, of 32 by the pipe's issue, against 24 of the mad.wide chains
+// (the field kernels reach 27).
 template <int MODE>
 __global__ void k_imad_peak(uint32_t seed, int iters, uint32_t *out)
 {
@@ -3233,14 +3236,17 @@ int hs_measure_imad_peak(hs_context *h, double *imad_per_s)
     Context &ctx = h->c;
     std::lock_guard<std::mutex> lk(ctx.mu);
     DeviceGuard g(ctx.device);
-    double pair = 0.0, wide = 0.0;
+    double pair = 0.0, wide = 0.0, hi = 0.0;
     int rc = imad_probe(ctx, 0, &pair);
     if (rc == HS_OK)
         rc = imad_probe(ctx, 1, &wide);
+    if (rc == HS_OK)
+        rc = imad_probe(ctx, 3, &hi);
     if (rc != HS_OK)
         return rc;
-    // a lo/hi pair is one product (2 IMAD-eq); a wide instruction is one product
-    *imad_per_s = std::max(pair, 2.0 * wide);
+    // a lo/hi pair is one product (2 IMAD-eq); a wide instruction is one product, and a
+    // mad.hi takes as long
+    *imad_per_s = std::max(pair, 2.0 * std::max(wide, hi));
     return HS_OK;
 }
 

@@ -358,9 +358,9 @@ int hs_profile_enable(hs_context *ctx, int on);
 int hs_profile_read(hs_context *ctx, double *accumulate_ms, uint64_t *accumulate_launches, uint64_t *entries,
                     int reset);
 /* Integer multiply throughput of this device: kernels of independent
- * mad.lo/mad.hi chains and of independent mad.wide.u32 chains on every SM,
- * timed with CUDA events.  Returns the faster, in IMAD-equivalents per second
- * (a 32x32->64 product counts as 2, in either form). */
+ * mad.lo/mad.hi, mad.wide.u32 and mad.hi chains on every SM, timed with CUDA
+ * events.  Returns the fastest, in IMAD-equivalents per second (a 32x32->64
+ * product counts as 2 in either form; a mad.hi holds the pipe as long as one). */
 int hs_measure_imad_peak(hs_context *ctx, double *imad_per_s);
 /* The probes behind hs_measure_imad_peak, in instructions per second over the
  * whole device: rates[0] mad.lo/mad.hi alternating (each instruction is one

@@ -106,3 +106,42 @@ def test_decompress_device(ctx, curve):
     want, nbad = oracle.decompress(curve, enc.reshape(-1))
     assert d_out.cpu().numpy().tobytes() == want.tobytes()
     assert int((d_valid.cpu().numpy() == 0).sum()) == nbad
+
+
+def test_multiply_peak_is_not_below_what_decoding_reaches(ctx):
+    """the peak that the bench quotes its fractions against, beside the multiplications
+    that decoding executes (counted in the bench)"""
+    import sys
+
+    import torch
+
+    import helioselene_gb300 as hs
+    from conftest import ROOT
+    sys.path.insert(0, str(ROOT))
+    import bench
+    n = 1 << 18
+    peak = ctx.measure_imad_peak()
+    g = torch.Generator(device="cuda:0")
+    g.manual_seed(3)
+    u = torch.randint(0, 128, (n, 32), dtype=torch.uint8, device="cuda:0", generator=g)
+    pts = torch.empty(n, 64, dtype=torch.uint8, device="cuda:0")
+    out, valid = torch.empty_like(pts), torch.empty(n, dtype=torch.uint8, device="cuda:0")
+    stream = torch.cuda.ExternalStream(ctx.stream)
+    for curve in (0, 1):
+        torch.cuda.synchronize()
+        ctx.map_to_curve_device(curve, u.data_ptr(), n, pts.data_ptr())
+        stream.synchronize()
+        enc = pts[:, :32].clone()
+        enc[:, 31] |= (pts[:, 32] & 1) << 7
+        torch.cuda.synchronize()
+        ms = []
+        for _ in range(4):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record(stream)
+            ctx.decompress_device(curve, enc.data_ptr(), n, out.data_ptr(), valid.data_ptr())
+            b.record(stream)
+            stream.synchronize()
+            ms.append(a.elapsed_time(b))
+        assert bool(valid.all()) and torch.equal(out, pts)
+        work = n * (bench.DECODE_SQR[curve] * bench.EXEC_SQR[curve] + bench.DECODE_MUL[curve] * bench.EXEC_MUL[curve])
+        assert work / (min(ms) * 1e-3) < peak
