@@ -1762,10 +1762,13 @@ int execute_batch(Context &ctx, const BatchPlan &p, const BatchBuffers &b, void 
     }
     // The descriptors of a captured shape live in a buffer owned by the graph:
     // uploaded once here, so a replay needs no host copy (a pageable copy
-    // would synchronise the stream).
+    // would synchronise the stream).  The upload is on the stream that the graph is
+    // launched on: cudaMemcpy from pageable memory may return before the device has
+    // the data, and a non-blocking stream does not wait for the default one.
     GraphEntry ent;
     HS_CU(cudaMalloc(&ent.d_desc, (size_t)p.M * sizeof(MsmDesc)), "descriptor allocation");
-    cudaError_t ue = cudaMemcpy(ent.d_desc, p.msms.data(), (size_t)p.M * sizeof(MsmDesc), cudaMemcpyHostToDevice);
+    cudaError_t ue = cudaMemcpyAsync(ent.d_desc, p.msms.data(), (size_t)p.M * sizeof(MsmDesc), cudaMemcpyHostToDevice,
+                                     st);
     if (ue != cudaSuccess) {
         cudaFree(ent.d_desc);
         return fail(ctx, ue, "descriptor upload");
@@ -2112,7 +2115,7 @@ static int execute_split(Context &ctx, const SplitPlan &s, const void *d_scalars
     GraphEntry ent;
     HS_CU(cudaMalloc(&ent.d_desc, 2 * sizeof(MsmDesc)), "descriptor allocation");
     const MsmDesc both[2] = {s.hi.msms[0], s.lo.msms[0]};
-    cudaError_t ue = cudaMemcpy(ent.d_desc, both, sizeof(both), cudaMemcpyHostToDevice);
+    cudaError_t ue = cudaMemcpyAsync(ent.d_desc, both, sizeof(both), cudaMemcpyHostToDevice, st);  // as in execute_batch
     if (ue != cudaSuccess) {
         cudaFree(ent.d_desc);
         return fail(ctx, ue, "descriptor upload");
@@ -2614,11 +2617,12 @@ static int msm_host(Context &ctx, int curve, const uint8_t *lead_scalar, const v
             if (g.key == key)
                 hit = &g;
         if (!hit) {
-            // descriptors in a buffer owned by the graph, uploaded once here
+            // descriptors in a buffer owned by the graph, uploaded once here (on the
+            // graph's stream, as in execute_batch)
             GraphEntry ent;
             HS_CU(cudaMalloc(&ent.d_desc, 2 * sizeof(MsmDesc)), "descriptor allocation");
             const MsmDesc both[2] = {p0.msms[0], split ? s.lo.msms[0] : p0.msms[0]};
-            cudaError_t ue = cudaMemcpy(ent.d_desc, both, sizeof(both), cudaMemcpyHostToDevice);
+            cudaError_t ue = cudaMemcpyAsync(ent.d_desc, both, sizeof(both), cudaMemcpyHostToDevice, st);
             if (ue != cudaSuccess) {
                 cudaFree(ent.d_desc);
                 return fail(ctx, ue, "descriptor upload");

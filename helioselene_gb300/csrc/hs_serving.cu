@@ -604,7 +604,11 @@ int hs_server_set_pool(hs_server *h, int curve, const void *pts, size_t n)
         p.d = nullptr;
         return HS_ENOMEM;
     }
-    if (cudaMemcpy(p.d, pts, n * 64, cudaMemcpyHostToDevice) != cudaSuccess) {
+    // on a slot's stream and waited for: the slots' streams do not wait for the default
+    // one, on which cudaMemcpy may return before the device has the data
+    cudaStream_t st = S.slots[0]->ctx.stream;
+    if (cudaMemcpyAsync(p.d, pts, n * 64, cudaMemcpyHostToDevice, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess) {
         cudaGetLastError();
         return HS_ECUDA;
     }

@@ -56,3 +56,16 @@ def test_host_only_calls(lib):
     assert lib.hs_msm(None, 0, None, None, 0, 0, None, 0) == -1
     lib.hs_context_create.restype = ctypes.c_int
     assert lib.hs_context_create(None, 0) == -1
+
+
+def test_uploads_are_ordered_on_a_stream():
+    """cudaMemcpy from pageable memory and cudaMemset may return before the device is done,
+    and the library's streams do not wait for the default stream: every upload names a
+    stream (a blocking cudaMemcpy is for reading back)"""
+    bad = []
+    for src in sorted((ROOT / "helioselene_gb300" / "csrc").glob("*.cu*")):
+        text = re.sub(r"//[^\n]*", "", src.read_text())
+        for m in re.finditer(r"\bcudaMem(?:cpy|set)(?:2D)?\s*\((?:[^()]|\((?:[^()]|\([^()]*\))*\))*\)", text):
+            if "cudaMemcpyDeviceToHost" not in m.group(0):
+                bad.append((src.name, " ".join(m.group(0).split())))
+    assert bad == []

@@ -88,3 +88,39 @@ def test_argument_checks(ctx):
     assert lib.hs_scalar_mul(h, 0, p, p, HS_AFF, 0, p, HS_AFF) == hs._lib.HS_OK          # n = 0: nothing to do
     assert lib.hs_context_set_priority(None, 1) == hs._lib.HS_EINVAL
     assert lib.hs_context_set_split(None, 0) == hs._lib.HS_EINVAL
+
+
+def test_first_calls_of_many_contexts_at_once():
+    """every call captures a launch sequence of its own, whose descriptors are uploaded
+    while the other contexts' uploads and kernels are under way"""
+    import torch
+
+    import helioselene_gb300 as hs
+    top = 20000
+    sc, pts, _ = oracle_inputs(0, top, seed=77)
+    d_s = torch.from_numpy(sc.reshape(-1).copy()).cuda()
+    d_p = torch.from_numpy(pts.reshape(-1).copy()).cuda()
+    jobs = [[(37 * i + 211 * k) % 5000 + (3000 if k % 3 else 14000) for k in range(12)] for i in range(12)]
+    d_o = torch.zeros(12, 12, 32, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+
+    def run(c, i):
+        for k, n in enumerate(jobs[i]):
+            c.msm_device(0, d_s.data_ptr() + 32 * k, d_p.data_ptr() + 64 * k, n, d_o[i, k].data_ptr(), HS_COMPRESSED)
+
+    ctxs = [hs.Context(0) for _ in range(12)]
+    ths = [threading.Thread(target=run, args=(c, i)) for i, c in enumerate(ctxs)]
+    [t.start() for t in ths]
+    [t.join() for t in ths]
+    torch.cuda.synchronize()
+    got = d_o.cpu().numpy().copy()
+    with hs.Context(0) as c:
+        c.set_graphs(False)
+        for i in range(12):
+            run(c, i)
+        torch.cuda.synchronize()
+    assert (got == d_o.cpu().numpy()).all()
+    k, n = 3, jobs[5][3]
+    assert got[5, k].tobytes() == oracle.msm(0, sc[k:k + n], pts[k:k + n])
+    for c in ctxs:
+        c.close()
