@@ -47,3 +47,22 @@ def test_commitments(own_ctx, curve, rounds, n, window, count):
     finally:
         own_ctx.default_batch_affine()
         fb.close()
+
+
+@pytest.mark.parametrize("curve", [0, 1])
+@pytest.mark.parametrize("n,window,count", [(17, 0, 300), (228, 0, 256), (620, 8, 200)])
+def test_every_commitment(own_ctx, curve, n, window, count):
+    """all results of the block sort against those of calls of fewer commitments, which
+    sort otherwise"""
+    _, G, _ = oracle_inputs(curve, n, seed=3 * n)
+    rng = np.random.default_rng(3 * n)
+    vals = rng.integers(0, 256, (count, n, 32), dtype=np.uint8)
+    vals[::9] = vals[::9, :1]
+    vals[4::9, ::2] = 0
+    fb = hs.FixedBase(own_ctx, curve, G, window=window)
+    try:
+        got = fb.commit(vals)
+        for lo in range(0, count, 100):
+            assert got[lo:lo + 100] == fb.commit(vals[lo:lo + 100]), lo
+    finally:
+        fb.close()

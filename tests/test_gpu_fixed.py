@@ -101,3 +101,30 @@ def test_tree_hash_layer_shapes(ctx, curve, n):
         assert fb.commit(vals) == want
     finally:
         fb.close()
+
+
+@pytest.mark.parametrize("curve", [0, 1])
+@pytest.mark.parametrize("n,window", [(300000, 16), (799999, 16), (800000, 20)])
+def test_default_width_of_large_generator_sets(curve, n, window):
+    """the table's width on both sides of its last border, and one dense commitment against
+    the same MSM without a table"""
+    import torch
+
+    import helioselene_gb300 as hs
+    g = torch.Generator(device="cuda:0")
+    g.manual_seed(n)
+    u = torch.randint(0, 128, (n, 32), dtype=torch.uint8, device="cuda:0", generator=g)
+    sc = torch.randint(0, 128, (n, 32), dtype=torch.uint8, device="cuda:0", generator=g)
+    pts = torch.empty(n, 64, dtype=torch.uint8, device="cuda:0")
+    out = torch.zeros(2, 32, dtype=torch.uint8, device="cuda:0")
+    torch.cuda.synchronize()
+    with hs.Context(0) as c:
+        c.map_to_curve_device(curve, u.data_ptr(), n, pts.data_ptr())
+        torch.cuda.synchronize()
+        fb = hs.FixedBase(c, curve, pts.cpu().numpy())
+        assert fb.window == window
+        fb.commit_device(sc.data_ptr(), 1, out[0].data_ptr(), hs.FMT_COMPRESSED)
+        c.msm_device(curve, sc.data_ptr(), pts.data_ptr(), n, out[1].data_ptr(), hs.FMT_COMPRESSED)
+        torch.cuda.synchronize()
+        fb.close()
+    assert (out[0] == out[1]).all() and out[0].any()

@@ -57,3 +57,19 @@ def test_scalar_mul_of_points_at_16_bytes(ctx, curve):
         torch.cuda.synchronize()
         got.append(out.cpu().numpy().tobytes())
     assert got[0] == got[1]
+
+
+@pytest.mark.parametrize("curve", [0, 1])
+@pytest.mark.parametrize("offset", [0, 16])
+def test_scalar_mul_of_points_at_16_bytes_against_the_oracle(ctx, curve, offset):
+    torch = pytest.importorskip("torch")
+    import oracle
+    sc, pts, _ = oracle_inputs(curve, 33, seed=6)
+    d_sc, d_pts = torch.from_numpy(sc.reshape(-1).copy()).to("cuda:0"), shifted(torch, pts.reshape(-1), offset)
+    out = torch.zeros(33 * 32, dtype=torch.uint8, device="cuda:0")
+    torch.cuda.synchronize()
+    ctx.scalar_mul_device(curve, d_sc.data_ptr(), d_pts.data_ptr(), 33, out.data_ptr(), hs.FMT_COMPRESSED)
+    torch.cuda.synchronize()
+    got = out.cpu().numpy().reshape(33, 32)
+    for i in range(33):
+        assert got[i].tobytes() == oracle.msm(curve, sc[i:i + 1], pts[i:i + 1]), i

@@ -232,3 +232,39 @@ def test_pools_and_rules_while_batches_are_launched(pools):
             t.join()
         assert changes[0] > 0
         srv.set_pool(0, pools[0])
+
+
+@pytest.mark.parametrize("curve", [0, 1])
+@pytest.mark.parametrize("window", [4, 8])
+def test_many_small_pool_only_requests_in_one_batch(pools, curve, window):
+    """hundreds of requests over the pool table in one launch sequence, a block each in the
+    sort: one point to the most a block takes, scalars that are zero, have every bit set
+    or put every point in one bucket, the same base again and again"""
+    import helioselene_gb300 as hs
+    rng = np.random.default_rng(13 + window)
+    most = {4: 315, 8: 620}[window]  # 20480 entries at 65 and 33 windows
+    sizes = [1, 2, most, 31, 32, 33] + [int(x) for x in rng.integers(1, most, 250)]
+    reqs = []
+    for i, n in enumerate(sizes):
+        s = rng.integers(0, 256, (n, 32), dtype=np.uint8)
+        if i % 7 == 1:
+            s[:] = s[0]
+        elif i % 7 == 2:
+            s[::2], s[1::2] = 0, 255
+        idx = rng.integers(0, 4096, n).astype(np.uint32)
+        if i % 7 == 3:
+            idx[:] = idx[0]
+        reqs.append((s, idx))
+    big = rng.integers(0, 128, (1 << 18, 32), dtype=np.uint8)
+    big_idx = rng.integers(0, 4096, 1 << 18).astype(np.uint32)
+    pts = np.concatenate([pools[curve][idx] for _, idx in reqs])
+    want = oracle.msm_many(curve, np.concatenate([s for s, _ in reqs]), pts, sizes)
+    with hs.Server(0, slots=1) as srv:
+        srv.set_pool_window(curve, window)
+        srv.set_pool(curve, pools[curve])
+        first = srv.submit(curve, big, big_idx)  # the slot is busy while the others are queued
+        tickets = [srv.submit(curve, s, idx) for s, idx in reqs]
+        srv.wait(first)
+        got = [srv.wait(t)[0] for t in tickets]
+        assert srv.stats()["max_batch_msms"] >= 128
+    assert [i for i, (g, w) in enumerate(zip(got, want)) if g != w] == []

@@ -115,3 +115,11 @@ def test_rounds_and_workspace_of_many_small_msms(plan, count, n, rounds):
 def test_every_chunk_of_commitments_has_its_workspace(plan, n, window, count, rounds):
     out = plan("chunks", n, window, count, rounds)
     assert len(out) >= 2 and set(out) == {"1"}, out
+
+
+# many MSMs of 600 points: 7 bits by default, more where that exceeds what is indexed
+@pytest.mark.parametrize("count,c,fits", [(96000, 7, 1), (97000, 8, 1), (130000, None, 0)])
+def test_widths_at_the_limit_of_the_entries(plan, count, c, fits):
+    got, entries, _, _, _, width = plan("batch", 0, 0, count, 600).split()
+    assert int(got) == fits and (c is None or (int(width) == 7 if c == 7 else int(width) >= c))
+    assert not fits or int(entries) < 2**31
