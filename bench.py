@@ -52,16 +52,15 @@ IMAD_PER_MODMUL = {0: 144, 1: 232}
 # instead of 64; a difference of two products shares one fold on F_q
 EXEC_MUL, EXEC_SQR, EXEC_MUL_SUB = {0: 144, 1: 192}, {0: 88, 1: 136}, {0: 288, 1: 320}
 # dram__bytes_read.sum + dram__bytes_write.sum of the bucket-accumulation phase of
-# one MSM at n = 2^20 (Helios, Selene), from ncu --set full captures of this
+# one MSM at n = 2^20 (Helios, Selene), from ncu captures of this
 # workload, by accumulation form (batch-affine rounds): 0 is k_accumulate, 1 is
 # k_ba_pairs + k_ba_invert + k_ba_finish + k_accumulate_level
 ACC_TRAFFIC = {
-    0: {"bytes": (477.2e6, 497.5e6), "capture": ("2026-12-04, commit 14d24da, k_accumulate",) * 2},
-    1: {"bytes": (2916.1e6, 2941.9e6),
-        "capture": ("2026-12-04, commit f0491f5, k_ba_pairs + k_ba_invert + k_ba_finish + k_accumulate_level",
-                    "2026-12-04, commit d2e236f, k_ba_pairs + k_ba_invert + k_ba_finish + k_accumulate_level")},
-    2: {"bytes": (None, 4316.5e6),
-        "capture": (None, "2026-12-04, commit f0491f5, two rounds of k_ba_pairs + k_ba_invert + k_ba_finish, "
+    0: {"bytes": (491.5e6, 489.9e6), "capture": ("2026-12-05, commit c6aa49e, k_accumulate",) * 2},
+    1: {"bytes": (2921.0e6, None),
+        "capture": ("2026-12-05, commit c6aa49e, k_ba_pairs + k_ba_invert + k_ba_finish + k_accumulate_level", None)},
+    2: {"bytes": (None, 4321.2e6),
+        "capture": (None, "2026-12-05, commit c6aa49e, two rounds of k_ba_pairs + k_ba_invert + k_ba_finish, "
                           "then k_accumulate_level")},
 }
 DEFAULT_BA_ROUNDS = (1, 2)  # the library's default accumulation form of device-resident MSMs (Helios, Selene)
