@@ -774,7 +774,8 @@ struct Field {
                 }
                 // no swap is due for (1 - D) / 2 steps: of these, up to six at once, by
                 // the multiple w f that clears as many low bits of g (the halvings
-                // are the next turn's even steps).  f (2 - f^2) = 1/f mod 64.
+                // are the next turn's even steps), a step known from the variable-time
+                // inversion of libsecp256k1.  f (2 - f^2) = 1/f mod 64.
                 int lim = (1 - D) >> 1;
                 lim = lim < left ? lim : left;
                 lim = lim < 6 ? lim : 6;

@@ -755,8 +755,8 @@ __global__ void __launch_bounds__(RED_QUADS * 4) k_window_sum(const uint4 *__res
 //     sum_t acc_t + m0 sum_t t run_t,   sum_t t run_t = sum_{t >= 1} sum_{h >= t} run_h.
 // Three additions per group and no scan, tree or barrier: where the windows fill the
 // device, this does with some 3 steps of a whole warp per window of 8 groups what
-// k_window_chunks' block per window did with 13.  Bound by the multiplier.  GB300: 4 x
-// 256 verification batches 2.10 -> 1.79 ms, 1024 MSMs of 64 to 65536 points 28.4 ->
+// k_window_chunks' block per window did with 13.  Bound by the multiplier.  GB300: 256
+// verifications (as many MSMs a curve) 2.10 -> 1.79 ms, 1024 MSMs of 64 to 65536 points 28.4 ->
 // 27.2 ms, 8192 commitments to 228 generators 7.02 -> 6.64 ms, 4096 x 64 points 6.33 |
 // 9.73 -> 4.28 | 6.98 ms (Helios | Selene).
 // The chain of 3 T additions has to be outweighed by the windows there are, 64 per group
@@ -937,7 +937,10 @@ __global__ void __launch_bounds__(128, 1) k_combine(const uint4 *__restrict__ S,
 // other's chains by more than the additions were worth (GB300, 64-point MSMs, Helios |
 // Selene, us: 19 of them 369 | 499 without groups, 360 | 488 with; 38 of them 423 |
 // 562 and 426 | 600).  With them one MSM of 16 points from host memory takes 267 us
-// instead of 289, 65521 encodings 945 instead of 962.
+// instead of 289, 65521 encodings 945 instead of 962.  By width, without and with (one
+// MSM, Helios | Selene, us): 33 windows of 8 bits 299 | 403 and 272 | 361; 26 of 10 bits
+// 475 | 626 and 452 | 593; 20 of 13 bits 559 | 730 and 544 | 707; 17 of 16 bits 841 | 1110
+// and 832 | 1115; 15 of 18 bits 1370 | 1935 and 1363 | 1927.
 static uint32_t combine_groups(const BatchPlan &p, int sm_count)
 {
     uint32_t wr = 1;
@@ -1246,12 +1249,12 @@ cudaError_t msm_tail(Context &ctx, const BatchPlan &p, const BatchBuffers &b)
             return launch_combine<C>(ctx, p, b, st);
         }
         // A plan of few chunks (one or a few MSMs) is latency-bound, and so are
-        // windows of at most 16 groups: one thread per group up to
-        // RED_CHUNK_THREADS groups.  Many chunks of more groups (a batch of larger
-        // MSMs) fill the device, and RED_CHUNK_Q groups per thread keep the scans'
-        // extra work small.  (Measured: 256 FCMP++ verifications, 16 groups per
-        // window, 51k -> 65k per second one group per thread; 1024 MSMs of
-        // 64..65536 points 1.5% faster with four.)
+        // windows of at most 16 groups: one quad per group up to RED_QUADS groups.
+        // Many chunks of more groups (a batch of larger MSMs) fill the device, and
+        // RED_CHUNK_Q groups per quad keep the scans' extra work small.  (Measured with
+        // one thread where a quad is now: 256 verifications, 16 groups per window, 51k ->
+        // 65k per second with one group each; 1024 MSMs of 64 to 65536 points 1.5% faster
+        // with four.)
         const int wide = p.CH <= 4u * (uint32_t)ctx.sm_count || p.max_T <= 16;
         const uint32_t t2 =
             std::max<uint32_t>(32, 4 * std::min<uint32_t>(RED_QUADS, wide ? p.max_T : p.max_T / RED_CHUNK_Q));

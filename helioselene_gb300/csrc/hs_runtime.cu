@@ -194,7 +194,7 @@ int choose_window(const Context &ctx, int curve, size_t n, Widths use)
 // The sort of a batch of small fixed-base MSMs, a block each (k_recode_block): for
 // plans whose every MSM has its buckets and its entries in a block's shared memory, and
 // of enough MSMs to fill the device.  (Variable-base MSMs, whose windows have buckets
-// of their own, gained nothing: 4 x 256 verification batches 2.10 ms without, 2.12 with;
+// of their own, gained nothing: 256 verifications 2.10 ms without, 2.12 with;
 // 1024 MSMs of 64 to 65536 points lost 7%.)
 static void plan_block_sort(BatchPlan &p)
 {
@@ -3276,7 +3276,10 @@ int hs_measure_imad_rates(hs_context *h, double rates[4])
 // window is as even as the others (8 commitments over 2^18 generators on GB300, ms,
 // Helios | Selene: 3.65 | 4.47 with 16, 4.07 | 5.18 with 18; 2^19: 6.77 | 8.69 with
 // 16, 7.73 | 9.70 with 18), and 20 bits, 13 windows for 16, pay from some 2^20
-// generators (6.83 | 9.28 at 2^19; 2^20: 13.4 | 17.5 with 16, 12.4 | 16.5 with 20).
+// generators (6.83 | 9.28 at 2^19; 2^20: 13.4 | 17.5 with 16, 12.4 | 16.5 with 20).  One
+// commitment by itself, whose buckets are reduced for it alone, would rather have 18 or
+// 20 bits from some 2^17 on (us: 2^19 1279 | 1608 with 16, 1043 | 1625 with 20; 2^17 552 |
+// 853 and 494 | 625 with 18); a set is laid out once for many.
 constexpr size_t FIXED_WIDE_MIN = 800000;
 
 static int fixed_window(size_t n)

@@ -220,9 +220,9 @@ int hs_msm_batch(hs_context *ctx, const hs_msm_desc *descs, size_t count, int po
  * follow those of MSM i-1 in d_scalars / d_points; d_out receives count
  * records of out_fmt.  One launch sequence serves the whole batch: recode and
  * counting sort over all MSMs' buckets, one accumulation launch, reductions
- * indexed by MSM, and one warp per MSM for the window combination.  Window
- * widths come from the context's rules (hs_context_set_window) or the cost
- * model, per MSM size.  Runs on the context stream; does not synchronise. */
+ * indexed by MSM, and a block (for few MSMs a cluster of blocks) per MSM for
+ * the window combination.  Window widths come from the context's rules
+ * (hs_context_set_window) or the built-in widths, per MSM size.  Runs on the context stream; does not synchronise. */
 int hs_msm_batch_device(hs_context *ctx, int curve, const size_t *sizes, size_t count, const void *d_scalars,
                         const void *d_points, void *d_out, int out_fmt);
 

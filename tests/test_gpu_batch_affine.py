@@ -1,5 +1,5 @@
 """Batch-affine bucket accumulation (hs_context_set_batch_affine): rounds of
-pairwise affine additions that share one inversion per 2048 additions, then an
+pairwise affine additions that share one inversion per 32768 additions, then an
 XYZZ fold.  Every result is compared bit for bit with the oracle and with the
 XYZZ accumulation of every entry (rounds = 0), on the cases the affine formula
 treats apart: equal bases in a bucket (doubling), a base and its negation

@@ -410,7 +410,7 @@ def test_host_parts_edge_cases(ctx, curve):
 @pytest.mark.parametrize("curve", [0, 1])
 @pytest.mark.parametrize("n", [300, 2000])
 def test_small_plan_heavy_buckets(ctx, curve, n):
-    """small plans run the eight-lane group kernels (accumulation, merges, window
+    """small plans run the four-lane quad kernels (accumulation, merges, window
     reduction): one base repeated with one scalar fills one bucket per window
     with hundreds of entries (many segments: group merges and the heavy-bucket
     path), P and -P with equal scalars cancel inside buckets, and equal points
