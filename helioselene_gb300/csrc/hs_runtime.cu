@@ -121,10 +121,10 @@ struct WindowStep {
 };
 // One MSM by itself is latency-bound up to some 2^16 points: fewer buckets shorten
 // the reduction by more than the added windows cost (Helios | Selene, us: 8192
-// points 335 | 459 with c = 8, 350 | 474 with 10; 16384 378 | 506 with 9, 426 | 559
-// with 11; 2^17 691 | 920 with 14, 718 | 947 with 13; 400000 1131 | 1534 with 14,
-// 1108 | 1512 with 16; 2^25 66.8 | 74.8 ms with 16, 63.4 | 69.4 with 20).  65536 points
-// take 543 | 716 with 13 and 537 | 707 with 14, but both curves' MSMs side by side 843
+// points 312 | 420 with c = 8, 334 | 444 with 10; 16384 361 | 475 with 9, 405 | 532
+// with 11; 2^17 693 | 914 with 14, 712 | 924 with 13; 400000 1132 | 1520 with 14,
+// 1109 | 1505 with 16; 2^25 66.8 | 74.8 ms with 16, 63.4 | 69.4 with 20).  65536 points
+// take 533 | 692 with 13 and 527 | 681 with 14, but both curves' MSMs side by side 843
 // and 892.
 static const WindowStep ALONE_WINDOWS[] = {{10000, 8},  {24000, 9},   {48000, 10},
                                            {80000, 13}, {350000, 14}, {size_t(1) << 24, 16}};
@@ -135,15 +135,15 @@ static const WindowStep ALONE_WINDOWS[] = {{10000, 8},  {24000, 9},   {48000, 10
 static const WindowStep DECODED_WINDOWS[] = {{10000, 8},   {24000, 9},   {40000, 10},          {90000, 12},
                                              {150000, 13}, {350000, 14}, {size_t(1) << 24, 16}};
 // MSMs of a batch fill the device together, so the operations count (ms: 1024 x 256
-// points 2.60 | 3.66 with c = 6, 2.97 | 4.51 with 8; 4096 x 64 6.23 | 9.31 with 5,
-// 10.0 | 15.8 with 8; 32 x 16384 1.67 | 2.24 with 10, 1.75 | 2.31 with 11; 16 x 65536
-// 2.61 | 3.45 with 12, 2.73 | 3.61 with 13; 2 x 2^19 2.21 | 2.93 with 14, 2.25 | 2.97
-// with 16, 2.37 | 3.13 with 15).
+// points 2.03 | 3.06 with c = 6, 2.48 | 3.81 with 8; 4096 x 64 4.04 | 6.35 with 5,
+// 7.99 | 13.1 with 8; 32 x 16384 1.67 | 2.26 with 10, 1.73 | 2.38 with 11; 16 x 65536
+// 2.60 | 3.48 with 12, 2.64 | 3.61 with 13; 2 x 2^19 2.21 | 2.92 with 14, 2.22 | 3.06
+// with 16, 2.34 | 3.11 with 15).
 static const WindowStep BATCH_WINDOWS[] = {{160, 5},    {500, 6},    {1600, 7},   {5000, 8},    {7000, 9},
                                            {24000, 10}, {90000, 12}, {200000, 13}, {700000, 14}, {size_t(1) << 24, 16}};
 // The narrow widths pay from about this many MSMs, whose 33 x 128 buckets of c = 8
-// the reduction would notice (64 points each, us: 64 MSMs 414 with c = 6, 482 with 8;
-// 8 MSMs 349 with 6, 330 with 8).
+// the reduction would notice (64 points each, us: 64 MSMs 393 | 525 with c = 6, 481 |
+// 664 with 8; 8 MSMs 297 | 389 with 6, 293 | 389 with 8).
 constexpr uint32_t NARROW_MIN_MSMS = 64;
 
 // the fewest additions: W(c) * (n * madd + 2^(c-1) * 2 adds), madd ~ 10 M, add ~ 14 M
@@ -296,8 +296,9 @@ static uint32_t seg_cap(uint64_t ent, uint64_t nb)
 // 2^21 points 4657 with one round, 4525 with two; 2^19 1762 and 1853; 2^18 1280 and
 // 1455); the MSMs of a batch, mostly beside the other curve's, keep theirs.
 // A bucket's list is padded to a multiple of 2 or 4, so sparse lists are mostly padding:
-// 4096 x 64 points in 32 buckets a window (2 entries each) 6835 us without, 7767 with
-// two; in 16 buckets (4 each) 6623 and 6992; 8192 x 200 in 32 (6 each) 19549 and 19321.
+// 4096 x 64 Selene points in 32 buckets a window (2 entries each) 6835 us without, 7767
+// with two; in 16 buckets (4 each) 6623 and 6992; 8192 x 200 in 32 (6 each) 19549 and
+// 19321.
 // And the workspace of many tiny MSMs would be mostly that of the rounds: 281073 of at
 // most 5 points 92 GB with two, 19 without.
 constexpr uint64_t BA_TWO_MIN_ENTRIES = uint64_t(1) << 23;
