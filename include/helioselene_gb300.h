@@ -94,7 +94,8 @@ void *hs_context_stream(hs_context *ctx);
  * the bucket loop both replace).  Results are identical either way.  Default:
  * one round on Helios and two on Selene, from 7 * 2^20 entries (2^21 for the
  * halves of a split MSM and for a server's slots; one round for a lone MSM or a
- * half of fewer than 2^23), except in two kinds of plans where a curve's MSMs
+ * half of fewer than 2^23; none in variable-base plans of fewer than five
+ * entries per bucket), except in two kinds of plans where a curve's MSMs
  * mostly run alone: fixed-base commitments take none on Helios and two on
  * Selene (from 2^21 entries), single MSMs from host buffers none and one,
  * until this call sets the curve.  rounds = -1 restores the defaults.  Host-input calls
@@ -222,7 +223,9 @@ int hs_msm_batch(hs_context *ctx, const hs_msm_desc *descs, size_t count, int po
  * counting sort over all MSMs' buckets, one accumulation launch, reductions
  * indexed by MSM, and a block (for few MSMs a cluster of blocks) per MSM for
  * the window combination.  Window widths come from the context's rules
- * (hs_context_set_window) or the built-in widths, per MSM size.  Runs on the context stream; does not synchronise. */
+ * (hs_context_set_window) or the built-in widths, per MSM size.  HS_ERANGE when
+ * the batch's (point, window) entries or its buckets reach 2^31.  Runs on the
+ * context stream; does not synchronise. */
 int hs_msm_batch_device(hs_context *ctx, int curve, const size_t *sizes, size_t count, const void *d_scalars,
                         const void *d_points, void *d_out, int out_fmt);
 
@@ -315,7 +318,8 @@ int hs_server_set_pool_window(hs_server *srv, int curve, int window);
  * clears the curve's rules); applies to batches planned after the call */
 int hs_server_set_window(hs_server *srv, int curve, size_t n_min, size_t n_max, int window);
 /* queue a request; HS_ERANGE if it alone exceeds the batch caps or the budget,
- * or its n x windows reaches 2^31 (batches are also formed below that bound) */
+ * or its n x windows reaches 2^31 (batches are also formed below that bound, of
+ * entries and of buckets) */
 int hs_server_submit(hs_server *srv, const hs_request *req, uint64_t *ticket);
 /* wait up to timeout_ms for a request: HS_OK (result written, latency from
  * submit to completion in *latency_ms), HS_ETIMEDOUT, or the failure status */
